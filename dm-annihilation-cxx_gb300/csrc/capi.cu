@@ -30,6 +30,7 @@ struct DevBuf {
 struct RingTables {
     double *z = nullptr, *st = nullptr, *theta = nullptr, *step = nullptr;
     float *st32 = nullptr, *step32 = nullptr;
+    float2 *th2 = nullptr;
 };
 
 }  // namespace
@@ -44,7 +45,10 @@ struct Work {
     // segmented render (disc_seg.cu): work items, per-disc item ranges,
     // weight sums and pixel counts, and the FP32 deposit plane
     DevBuf seg_items, seg_sorted, seg_cls, seg_first, seg_nit, seg_S, seg_px, plane32;
-    bool seg_plane = false;   // plane32 holds a zeroed plane for the open map
+    bool plane_clean = false;   // plane32 is all zero (every segment's flush leaves it so)
+    // tiled render (disc_tile.cu): the pair list, its histogram and ranges,
+    // the work units, the general discs
+    DevBuf tile_hdr, tile_list, tile_hist, tile_base, tile_units, tile_gen;
 };
 
 struct dmann_ctx {
@@ -275,6 +279,13 @@ dmann_status ring_tables(dmann_ctx *ctx, int nside, RingTables &out) {
     CK(cudaMemcpy(t.st32, st32.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
     CK(cudaMalloc(&t.step32, sizeof(float) * n));
     CK(cudaMemcpy(t.step32, stp32.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
+    std::vector<float2> th2(n);
+    for (int r = 0; r < n; r++) {
+        th2[r].x = (float)th[r];
+        th2[r].y = (float)(th[r] - (double)th2[r].x);
+    }
+    CK(cudaMalloc(&t.th2, sizeof(float2) * n));
+    CK(cudaMemcpy(t.th2, th2.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
     ctx->rings[nside] = t;
     out = t;
     return DMANN_OK;
@@ -295,7 +306,7 @@ dmann_status collect_stats(dmann_ctx *ctx) {
         ctx->stats.disc_warp_ms = ctx->stats.disc_ms - ms;
     }
     ctx->stats.pass1_ms = ctx->stats.pass2_ms = 0.0;
-    if (ctx->seg_timed && ctx->h_ctr[C_SEG_MODE] == 1) {   // the last chunk was segmented
+    if (ctx->seg_timed && ctx->h_ctr[C_SEG_MODE] > 0) {   // the last chunk was tiled or segmented
         CK(cudaEventElapsedTime(&ms, ctx->evd0, ctx->evp1));
         ctx->stats.pass1_ms = ms;
         CK(cudaEventElapsedTime(&ms, ctx->evp1, ctx->evdm));
@@ -366,7 +377,8 @@ void dmann_destroy(dmann_ctx *ctx) {
     for (Work &wk : ctx->work) {
         DevBuf *wb[] = {&wk.theta, &wk.phi, &wk.ar, &wk.flux, &wk.cpix, &wk.key, &wk.queue, &wk.hist,
                         &wk.ctr, &wk.fsum, &wk.acc, &wk.chdr, &wk.seg_items, &wk.seg_sorted,
-                        &wk.seg_cls, &wk.seg_first, &wk.seg_nit, &wk.seg_S, &wk.seg_px, &wk.plane32};
+                        &wk.seg_cls, &wk.seg_first, &wk.seg_nit, &wk.seg_S, &wk.seg_px, &wk.plane32,
+                        &wk.tile_hdr, &wk.tile_list, &wk.tile_hist, &wk.tile_base, &wk.tile_units, &wk.tile_gen};
         for (DevBuf *b : wb)
             if (b->p) cudaFree(b->p);
     }
@@ -383,6 +395,7 @@ void dmann_destroy(dmann_ctx *ctx) {
         cudaFree(kv.second.step);
         cudaFree(kv.second.st32);
         cudaFree(kv.second.step32);
+        cudaFree(kv.second.th2);
     }
     if (ctx->h_ctr) cudaFreeHost(ctx->h_ctr);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -654,43 +667,103 @@ Accum make_accum(dmann_ctx *ctx) {
     return acc;
 }
 
-// The compensated form's block-class discs in work items and segments
-// (disc_seg.cu), then the warp class with the per-disc kernel.  The item
-// list holds up to 4 N + 2^20 items; the device decides per chunk whether
-// the segmented render or the per-disc block kernel (FP64 deposits) takes
-// the block class, and both are launched -- the one not chosen returns at
-// once -- so nothing here waits for the device and the sequence can be
-// captured in a graph.  Needs the disc headers, the FP32 plane and the item
-// buffers; without them `used` stays false and the caller renders with the
-// per-disc kernels alone.
 // Item slots of the segmented render: 4 n + 2^20 (items are indexed as int).
 size_t seg_capacity(size_t n) {
     return std::min<size_t>(4 * (n > 0 ? n : 1) + ((size_t)1 << 20), (size_t)0x7fffffff);
 }
 
-// The segmented render's buffers for chunks of n particles (optional: false
-// when an allocation fails; nothing is allocated when they are big enough).
-bool reserve_seg(dmann_ctx *ctx, size_t n) {
-    const size_t n1 = n > 0 ? n : 1, cap = seg_capacity(n);
-    return ensure_opt(ctx->w->seg_first, 8 * n1) && ensure_opt(ctx->w->seg_nit, 4 * n1) &&
-           ensure_opt(ctx->w->seg_S, 8 * n1) && ensure_opt(ctx->w->seg_px, 8 * n1) &&
-           ensure_opt(ctx->w->seg_cls, kSegBufBytes) && ensure_opt(ctx->w->seg_items, 8 * cap) &&
-           ensure_opt(ctx->w->seg_sorted, 8 * cap);
+// Pair list slots of the tiled render: every disc in every tile where that
+// is little (then no chunk can exceed it), else 96 per particle and 2^24 (a
+// disc of the 16M set at Nside 2048 touches 33 tiles, one of the 134M set at
+// Nside 4096 about 55; chunks with more pairs are segmented).
+size_t tile_pairs_bound(size_t n, int nside) {
+    return (n > 0 ? n : 1) * (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
+}
+size_t tile_capacity(size_t n, int nside) {
+    return std::min(tile_pairs_bound(n, nside), 96 * n + ((size_t)1 << 24));
+}
+size_t tile_unit_capacity(size_t n, int nside) {
+    return tile_capacity(n, nside) / kUnitMax + 2 * (size_t)kUnitTarget +
+           (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
 }
 
-dmann_status render_segmented(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning &tu, size_t N,
-                              bool &used, bool timed = true) {
+// The buffers of the two large-chunk renders for chunks of n particles at
+// one Nside: grown when grow is set (a failed allocation is not an error: the
+// chunk takes a render that does without), else only looked at, as under
+// graph capture.
+bool have_opt(DevBuf &b, size_t bytes, bool grow) { return grow ? ensure_opt(b, bytes) : b.bytes >= bytes; }
+
+bool have_tile(dmann_ctx *ctx, size_t n, int nside, bool grow) {
+    Work &w = *ctx->w;
+    const size_t n1 = n > 0 ? n : 1, nt = (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
+    return have_opt(w.seg_S, 8 * n1, grow) && have_opt(w.seg_px, 8 * n1, grow) &&
+           have_opt(w.seg_cls, kSegBufBytes, grow) && have_opt(w.tile_gen, 4 * n1, grow) && have_opt(w.tile_hdr, sizeof(TileHdr) * n1, grow) &&
+           have_opt(w.tile_hist, 3 * nt * kTileClasses * sizeof(unsigned), grow) &&
+           have_opt(w.tile_base, 3 * nt * sizeof(long long), grow) &&
+           have_opt(w.tile_units, 3 * tile_unit_capacity(n, nside) * sizeof(TileUnit), grow) &&
+           have_opt(w.tile_list, 4 * tile_capacity(n, nside), grow);
+}
+
+// (the FP32 plane is zeroed here, on the context's stream, when it is new)
+bool have_seg(dmann_ctx *ctx, size_t n, int nside, bool grow) {
+    Work &w = *ctx->w;
+    const size_t n1 = n > 0 ? n : 1, cap = seg_capacity(n), P = 12 * (size_t)nside * (size_t)nside;
+    if (!(have_opt(w.seg_first, 8 * n1, grow) && have_opt(w.seg_nit, 4 * n1, grow) &&
+          have_opt(w.seg_S, 8 * n1, grow) && have_opt(w.seg_px, 8 * n1, grow) &&
+          have_opt(w.seg_cls, kSegBufBytes, grow) && have_opt(w.seg_items, 8 * cap, grow) &&
+          have_opt(w.seg_sorted, 8 * cap, grow)))
+        return false;
+    if (w.plane32.bytes < 4 * P) w.plane_clean = false;
+    if (!have_opt(w.plane32, 4 * P, grow)) return false;
+    if (!w.plane_clean && grow)
+        w.plane_clean = cudaMemsetAsync(w.plane32.p, 0, w.plane32.bytes, ctx->stream) == cudaSuccess;
+    return w.plane_clean;
+}
+
+// A chunk of n particles that may be too large for the per-disc kernels: the
+// estimates of its discs, at most npix each, can reach the threshold.
+bool may_be_large(size_t n, int nside, const dmann_tuning &tu) {
+    const int lg = tu.seg_min_deposits_log2 > 0 ? tu.seg_min_deposits_log2 : 28;
+    return (double)n * 12.0 * nside * nside >= std::ldexp(1.0, lg);
+}
+bool tile_always_fits(size_t n, int nside) { return tile_capacity(n, nside) == tile_pairs_bound(n, nside); }
+
+bool reserve_large(dmann_ctx *ctx, size_t n, int nside, const dmann_tuning &tu) {
+    if (!may_be_large(n, nside, tu)) return true;
+    const bool tile = have_tile(ctx, n, nside, true);
+    return (tile && tile_always_fits(n, nside)) || have_seg(ctx, n, nside, true) || tile;
+}
+
+// The compensated form's block-class discs of a chunk that may be large:
+// the device counts its (disc, tile) pairs and decides per chunk between the
+// tiled render (disc_tile.cu), the segmented render (disc_seg.cu: chunks
+// whose pairs the list does not hold) and the per-disc block kernel (FP64
+// deposits).  All that are possible are launched, those not chosen return at
+// once, so nothing here waits for the device and the sequence can be captured
+// in a graph; then the warp class with the per-disc kernel.  Needs the disc
+// headers; `used` stays false (the caller renders with the per-disc kernels
+// alone) without them or the buffers, and for chunks that cannot be large: a
+// call of a few thousand particles launches 3 kernels here instead of 20, or
+// 150 with the segments' slots.
+dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning &tu, size_t N,
+                          bool &used, bool grow = true) {
     used = false;
-    if (!da.chdr || !ctx->w->seg_plane || !reserve_seg(ctx, N)) return DMANN_OK;
-    const size_t cap = seg_capacity(N);
+    const bool timed = grow;
+    const int nside = ctx->g.nside;
+    if (!da.chdr || !may_be_large(N, nside, tu)) return DMANN_OK;
+    Work &w = *ctx->w;
+    const bool tile = have_tile(ctx, N, nside, grow);
+    const bool seg = !(tile && tile_always_fits(N, nside)) && have_seg(ctx, N, nside, grow);
+    if (!tile && !seg) return DMANN_OK;
     cudaStream_t s = ctx->stream;
     const int bt = tu.block_threads == 128 ? 128 : 256;
     const int lg = tu.seg_min_deposits_log2 > 0 ? tu.seg_min_deposits_log2 : 28;
-    char *buf = (char *)ctx->w->seg_cls.p;
+    char *buf = (char *)w.seg_cls.p;
     SegArgs sg{};
-    sg.items = (int2 *)ctx->w->seg_items.p;
-    sg.sorted = (int2 *)ctx->w->seg_sorted.p;
-    sg.cap = (long long)cap;
+    sg.items = (int2 *)w.seg_items.p;
+    sg.sorted = (int2 *)w.seg_sorted.p;
+    sg.cap = seg ? (long long)seg_capacity(N) : 0;
+    sg.pair_cap = tile ? (long long)tile_capacity(N, nside) : 0;
     sg.cls = (int *)buf;
     sg.cls_px = (long long *)(buf + kSegClsBytes);
     sg.seg_next = (unsigned long long *)(buf + kSegClsBytes + kSegClsPxBytes);
@@ -698,28 +771,52 @@ dmann_status render_segmented(dmann_ctx *ctx, const DiscArgs &da, const dmann_tu
     sg.ctl = (int *)(buf + kSegClsBytes + kSegClsPxBytes + kSegNextBytes + kSegSpanBytes);
     sg.min_est = 1LL << lg;
     sg.budget = (long long)ctx->g.npix * kDepPerPix;
-    sg.disc_first = (long long *)ctx->w->seg_first.p;
-    sg.disc_nitems = (int *)ctx->w->seg_nit.p;
-    sg.disc_S = (double *)ctx->w->seg_S.p;
-    sg.disc_px = (long long *)ctx->w->seg_px.p;
-    sg.plane = (float *)ctx->w->plane32.p;
+    sg.disc_first = (long long *)w.seg_first.p;
+    sg.disc_nitems = (int *)w.seg_nit.p;
+    sg.disc_S = (double *)w.seg_S.p;
+    sg.disc_px = (long long *)w.seg_px.p;
+    sg.plane = (float *)w.plane32.p;
+    TileArgs tg{};
+    tg.ctl = sg.ctl;
+    tg.nstrips = tile_strips(nside);
+    tg.ncol = tile_cols(nside);
+    tg.list = (unsigned *)w.tile_list.p;
+    tg.hist = (unsigned *)w.tile_hist.p;
+    tg.base = (long long *)w.tile_base.p;
+    tg.units = (TileUnit *)w.tile_units.p;
+    tg.unit_cap = (long long)tile_unit_capacity(N, nside);
+    tg.disc_S = sg.disc_S;
+    tg.disc_px = sg.disc_px;
+    tg.gen = (int *)w.tile_gen.p;
+    tg.hdr = (TileHdr *)w.tile_hdr.p;
     CK(cudaMemsetAsync(buf, 0, kSegBufBytes, s));
+    if (tile)
+        CK(cudaMemsetAsync(w.tile_hist.p, 0, 3 * (size_t)tg.nstrips * tg.ncol * kTileClasses * sizeof(unsigned), s));
     CK(launch_hdr(da, ctx->num_sms, s));
     CK(launch_seg_count(da, sg, bt, ctx->num_sms, s));
-    CK(launch_seg_norm(da, sg, bt, ctx->num_sms, tu.blocks_per_sm, s));
+    if (tile) CK(launch_tile_hdr(da, tg, seg, ctx->num_sms, s));
+    CK(launch_seg_decide(da, sg, s));
+    ctx->launches += 8;   // prep, scan, scatter, headers, counts, mode, block kernel, warp class
+    if (seg) CK(launch_seg_norm(da, sg, bt, ctx->num_sms, tu.blocks_per_sm, s));
+    if (tile) CK(launch_tile_norm(da, tg, ctx->num_sms, s));
     if (timed) CK(cudaEventRecord(ctx->evp1, s));
-    CK(launch_seg_sort(da, sg, ctx->num_sms, s));
-    CK(launch_seg_deposits(da, sg, bt, ctx->num_sms, tu.blocks_per_sm, ctx->g.npix, s));
+    if (tile) {
+        CK(launch_tile_deposits(da, tg, ctx->num_sms, s));
+        ctx->launches += 10 + (seg ? 1 : 0);
+    }
+    if (seg) {
+        w.plane_clean = false;
+        CK(launch_seg_sort(da, sg, ctx->num_sms, s));
+        CK(launch_seg_deposits(da, sg, bt, ctx->num_sms, tu.blocks_per_sm, ctx->g.npix, s));
+        w.plane_clean = true;
+        ctx->launches += 6 + 2 * kSegSlots;   // fill, pass 1, octaves, scan, sort, plan, slots
+    }
     DiscArgs db = da;
     db.block_skip = sg.ctl;
     CK(launch_disc_comp_block(db, ctx->num_sms, tu.blocks_per_sm, tu.block_threads, s));
     if (timed) CK(cudaEventRecord(ctx->evdm, s));
     CK(launch_disc_comp_warp(da, ctx->num_sms, s));
     if (timed) ctx->seg_timed = true;
-    // prep, scan, scatter, headers, item count, mode, item fill, pass 1,
-    // octave histogram, scan, sort, plan, kSegSlots x (deposits, flush),
-    // per-disc block kernel, warp class
-    ctx->launches += 14 + 2 * kSegSlots;
     used = true;
     return DMANN_OK;
 }
@@ -755,10 +852,6 @@ dmann_status dmann_map_begin(dmann_ctx *ctx, int nside, int precision) {
     CK(cudaMemsetAsync(ctx->w->acc.p, 0, 8 * P, s));
     CK(cudaMemsetAsync(ctx->w->ctr.p, 0, 8 * C_COUNT, s));
     CK(cudaMemsetAsync(ctx->w->fsum.p, 0, 8, s));
-    // the segmented render's FP32 plane: zero at the start of a map, and
-    // every segment's flush leaves it zero
-    ctx->w->seg_plane = precision == DMANN_COMP_F32 && ensure_opt(ctx->w->plane32, 4 * P);
-    if (ctx->w->seg_plane) CK(cudaMemsetAsync(ctx->w->plane32.p, 0, 4 * P, s));
     ctx->stats = dmann_stats{};
     ctx->launches = 0;
     ctx->disc_timed = false;
@@ -841,7 +934,7 @@ dmann_status dmann_map_add_v(dmann_ctx *ctx, const float *x, const float *y, con
     DiscArgs da;
     da.g = ctx->g;
     da.f = f;
-    da.rt = {ctx->rt.z, ctx->rt.st, ctx->rt.theta, ctx->rt.step, ctx->rt.st32, ctx->rt.step32};
+    da.rt = {ctx->rt.z, ctx->rt.st, ctx->rt.theta, ctx->rt.step, ctx->rt.st32, ctx->rt.step32, ctx->rt.th2};
     da.theta = pa.out.theta;
     da.phi = pa.out.phi;
     da.ar = pa.out.ar;
@@ -857,7 +950,7 @@ dmann_status dmann_map_add_v(dmann_ctx *ctx, const float *x, const float *y, con
         ctx->launches += 5;   // prep, scan, scatter, disc block, disc warp
     } else {
         bool seg = false;
-        if ((st = render_segmented(ctx, da, tu, N, seg)) != DMANN_OK) return st;
+        if ((st = render_large(ctx, da, tu, N, seg)) != DMANN_OK) return st;
         if (!seg) {
             CK(launch_disc_comp(da, ctx->num_sms, tu.blocks_per_sm, tu.block_threads, s, ctx->evdm));
             ctx->launches += 5 + (da.chdr ? 1 : 0);   // prep, scan, scatter, headers, block, warp
@@ -983,7 +1076,7 @@ dmann_status issue_observer(dmann_ctx *ctx, const float *const dev[6], int n, in
         DiscArgs da;
         da.g = ctx->g;
         da.f = f;
-        da.rt = {rt.z, rt.st, rt.theta, rt.step, rt.st32, rt.step32};
+        da.rt = {rt.z, rt.st, rt.theta, rt.step, rt.st32, rt.step32, rt.th2};
         da.theta = pa.out.theta;
         da.phi = pa.out.phi;
         da.ar = pa.out.ar;
@@ -997,7 +1090,7 @@ dmann_status issue_observer(dmann_ctx *ctx, const float *const dev[6], int n, in
         } else {
             da.chdr = headers_for(ctx, (size_t)n);
             bool seg = false;
-            dmann_status st = render_segmented(ctx, da, tu, (size_t)n, seg, false);
+            dmann_status st = render_large(ctx, da, tu, (size_t)n, seg, false);
             if (st != DMANN_OK) return st;
             if (!seg) CK(launch_disc_comp(da, ctx->num_sms, tu.blocks_per_sm, tu.block_threads, s, nullptr));
         }
@@ -1073,11 +1166,10 @@ dmann_status dmann_render_batch(dmann_ctx *ctx, const float *x, const float *y, 
         // before any capture: the disc headers and the segmented render's
         // buffers (the render checks them again and allocates nothing when
         // they fit)
-        ctx->w->seg_plane = false;
         if (precision == DMANN_COMP_F32) {
             reserve_headers(ctx, n1);
-            ctx->w->seg_plane = ensure_opt(ctx->w->plane32, 4 * Pmax) && reserve_seg(ctx, N);
-            if (ctx->w->seg_plane) CK(cudaMemsetAsync(ctx->w->plane32.p, 0, 4 * Pmax, s));
+            for (int k = 0; k < n_obs; k++)
+                if (k == 0 || nside[k] != nside[k - 1]) reserve_large(ctx, N, nside[k], tuning_for(ctx, nside[k]));
         }
     }
     ctx->w = &ctx->work[0];
@@ -1123,7 +1215,7 @@ dmann_status dmann_render_batch(dmann_ctx *ctx, const float *x, const float *y, 
     put(&ctx->vel_to_cgs, sizeof ctx->vel_to_cgs);
     put(ctx->fcpos, sizeof ctx->fcpos);
     put(&lanes, sizeof lanes);
-    for (int L = 0; L < lanes; L++) put(&ctx->work[L].seg_plane, sizeof(bool));
+    for (int L = 0; L < lanes; L++) put(&ctx->work[L].plane_clean, sizeof(bool));
     for (int k = 0; k < n_obs; k++) put(&tuning_for(ctx, nside[k]), sizeof(dmann_tuning));
     double rot0[9], opos0[3];
     std::memcpy(rot0, ctx->rot, sizeof rot0);
@@ -1353,7 +1445,7 @@ dmann_status dmann_adjoint_v(dmann_ctx *ctx, const float *x, const float *y, con
     DiscArgs da;
     da.g = g;
     da.f = f;
-    da.rt = {rt.z, rt.st, rt.theta, rt.step, rt.st32, rt.step32};
+    da.rt = {rt.z, rt.st, rt.theta, rt.step, rt.st32, rt.step32, rt.th2};
     da.theta = pa.out.theta;
     da.phi = pa.out.phi;
     da.ar = pa.out.ar;

@@ -49,6 +49,7 @@ struct RingTab {
     const double *step;   // 2 pi / (pixels in the ring)
     const float *st32;    // st and step rounded to FP32 (the compensated form's
     const float *step32;  // per-ring set-up runs in FP32 where it can)
+    const float2 *th2;    // theta as a two-float (the tiled render; null where it cannot run)
 };
 
 __host__ __device__ inline int64_t ring_start(const Hpx &g, int ring) {

@@ -361,14 +361,15 @@ __device__ inline float g_far(float x, const Run &r) {
     return t * t;
 }
 
-// Weights of pixels jj = (j, j + 32) of run r; also sin(x) (x half the
-// azimuth offset), the haversine h of the distance and g = theta^2 / 4.
+// Exponents of 2 of the weights of pixels jj = (j, j + 32) of run r; also
+// sin(x) (x half the azimuth offset), the haversine h of the distance and
+// g = theta^2 / 4.
 // TX, TH >= 0 fix the polynomial tiers at compile time (the disc kernels
 // dispatch on the particle's tiers once, outside the pixel loops); -1 reads
 // them from e.
 template <int TX = -1, int TH = -1>
-__device__ __forceinline__ float2 weight2x(const Ext &e, const Run &r, float2 jj, float2 &sn_out,
-                                          float2 &h_out, float2 &g_out) {
+__device__ __forceinline__ float2 exponent2x(const Ext &e, const Run &r, float2 jj, float2 &sn_out,
+                                            float2 &h_out, float2 &g_out) {
     const int tier_x = TX >= 0 ? TX : e.tier_x;
     const int tier_h = TH >= 0 ? TH : e.tier_h;
     const float2 x = fma2(jj, f2(r.steph), f2(r.d0h));
@@ -407,10 +408,17 @@ __device__ __forceinline__ float2 weight2x(const Ext &e, const Run &r, float2 jj
         if (h.x > 0.5f) g.x = g_far(x.x, r);
         if (h.y > 0.5f) g.y = g_far(x.y, r);
     }
-    const float2 t = mul2(g, f2(e.nK));
     sn_out = sn;
     h_out = h;
     g_out = g;
+    return mul2(g, f2(e.nK));
+}
+
+// The weights themselves.
+template <int TX = -1, int TH = -1>
+__device__ __forceinline__ float2 weight2x(const Ext &e, const Run &r, float2 jj, float2 &sn_out,
+                                          float2 &h_out, float2 &g_out) {
+    const float2 t = exponent2x<TX, TH>(e, r, jj, sn_out, h_out, g_out);
     return make_float2(ex2_approx(t.x), ex2_approx(t.y));
 }
 
@@ -451,6 +459,25 @@ __device__ __forceinline__ float2 weight2(const Ext &e, const Run &r, float2 jj)
         float2 sn, h, g;
         return weight2x<TX, TH>(e, r, jj, sn, h, g);
     }
+}
+
+// nK e0 .. nK e4 of the exponent polynomial for a ring (A, B) of a disc with
+// tier_h th (three terms of G for th 0, five for th 1).
+__device__ inline void poly_coeffs(float A, float B, float nK, int th, float c[5]) {
+    const float a4 = th ? 4.0f / 35.0f : 0.0f, a5 = th ? 128.0f / 1575.0f : 0.0f;
+    // G_k = sum_n C(n, k) a_n A^(n-k)
+    const float G0 = fmaf(A, A * fmaf(A, fmaf(A, fmaf(A, a5, a4), 8.0f / 45.0f), 1.0f / 3.0f), A);
+    const float G1 = fmaf(A, fmaf(A, fmaf(A, fmaf(A, 5.0f * a5, 4.0f * a4), 24.0f / 45.0f), 2.0f / 3.0f), 1.0f);
+    const float G2 = fmaf(A, fmaf(A, fmaf(A, 10.0f * a5, 6.0f * a4), 24.0f / 45.0f), 1.0f / 3.0f);
+    const float G3 = fmaf(A, fmaf(A, 10.0f * a5, 4.0f * a4), 8.0f / 45.0f);
+    const float G4 = fmaf(A, 5.0f * a5, a4);
+    const float B2 = B * B, B3 = B2 * B, B4 = B2 * B2;
+    const float g1 = G1 * B, g2 = G2 * B2, g3 = G3 * B3;
+    c[0] = nK * G0;
+    c[1] = nK * g1;
+    c[2] = nK * fmaf(g1, -1.0f / 3.0f, g2);
+    c[3] = nK * fmaf(g2, -2.0f / 3.0f, fmaf(g1, 2.0f / 45.0f, g3));
+    c[4] = nK * fmaf(G4, B4, fmaf(g2, 0.2f, fmaf(g1, -1.0f / 315.0f, -g3)));
 }
 
 // The double of a float f >= 0 from its bit pattern, with integer operations

@@ -1,5 +1,7 @@
 // disc_seg.cu -- the compensated-FP32 render of the block-class discs in
-// work items and segments.
+// work items and segments: for chunks whose (disc, tile) pairs the tiled
+// render's list does not hold (disc_tile.cu, about twice as fast).  Its
+// memory does not grow with the discs' areas.
 //
 // Work items.  Each disc of the block class (queue slots [0, nblk), the
 // largest discs) is cut into items of at most RCH rings (the block shape's
@@ -60,9 +62,9 @@
 // sequence reads the chunk's mode
 // (k_seg_decide) and returns at once when it has nothing to do, so the
 // whole render is one stream of launches with no host synchronisation.
-// Chunks too small for the L2 reduction rate to matter (a tunable threshold
-// on the estimated deposits), or with more work items than the item buffers
-// hold, take the per-disc kernels with FP64 deposits instead.
+// Chunks below a tunable threshold on the estimated deposits, or with more
+// work items than the item buffers hold, take the per-disc kernels with FP64
+// deposits instead.
 #include "comp_engine.cuh"
 
 namespace dmann {
@@ -92,25 +94,6 @@ struct SegSmem {
     int next_run;           // rings claimed so far (dynamic claims of the walk)
     int item;               // the claimed item
 };
-
-// nK e0 .. nK e4 of the exponent polynomial for a ring (A, B) of a disc with
-// tier_h th (three terms of G for th 0, five for th 1).
-__device__ inline void poly_coeffs(float A, float B, float nK, int th, float c[5]) {
-    const float a4 = th ? 4.0f / 35.0f : 0.0f, a5 = th ? 128.0f / 1575.0f : 0.0f;
-    // G_k = sum_n C(n, k) a_n A^(n-k)
-    const float G0 = fmaf(A, A * fmaf(A, fmaf(A, fmaf(A, a5, a4), 8.0f / 45.0f), 1.0f / 3.0f), A);
-    const float G1 = fmaf(A, fmaf(A, fmaf(A, fmaf(A, 5.0f * a5, 4.0f * a4), 24.0f / 45.0f), 2.0f / 3.0f), 1.0f);
-    const float G2 = fmaf(A, fmaf(A, fmaf(A, 10.0f * a5, 6.0f * a4), 24.0f / 45.0f), 1.0f / 3.0f);
-    const float G3 = fmaf(A, fmaf(A, 10.0f * a5, 4.0f * a4), 8.0f / 45.0f);
-    const float G4 = fmaf(A, 5.0f * a5, a4);
-    const float B2 = B * B, B3 = B2 * B, B4 = B2 * B2;
-    const float g1 = G1 * B, g2 = G2 * B2, g3 = G3 * B3;
-    c[0] = nK * G0;
-    c[1] = nK * g1;
-    c[2] = nK * fmaf(g1, -1.0f / 3.0f, g2);
-    c[3] = nK * fmaf(g2, -2.0f / 3.0f, fmaf(g1, 2.0f / 45.0f, g3));
-    c[4] = nK * fmaf(G4, B4, fmaf(g2, 0.2f, fmaf(g1, -1.0f / 315.0f, -g3)));
-}
 
 template <int BT>
 struct Blk {
@@ -328,7 +311,7 @@ __device__ inline void norm_item(const DiscArgs &a, SegSmem<RCH> &sm, int r0, in
 
 template <int BT, int RCH, int MINB>
 __global__ void __launch_bounds__(BT, MINB) k_seg_norm(DiscArgs a, SegArgs sg) {
-    if (sg.ctl[0] == 0) return;
+    if (sg.ctl[0] != 1) return;
     __shared__ SegSmem<RCH> sm;
     int2 it;
     const long long n_items = a.ctr[C_SEG_ITEMS];
@@ -373,7 +356,7 @@ __device__ inline void dep_item(const DiscArgs &a, SegSmem<RCH> &sm, int r0, int
 // returns at once when the plan has fewer segments.
 template <int BT, int RCH, int MINB>
 __global__ void __launch_bounds__(BT, MINB) k_seg_dep(DiscArgs a, SegArgs sg, int seg) {
-    if (sg.ctl[0] == 0 || seg >= sg.ctl[1]) return;
+    if (sg.ctl[0] != 1 || seg >= sg.ctl[1]) return;
     __shared__ SegSmem<RCH> sm;
     const SegSpan sp = sg.spans[seg];
     int2 it;
@@ -430,6 +413,7 @@ __global__ void __launch_bounds__(256) k_seg_count(DiscArgs a, SegArgs sg) {
             sg.disc_px[q] = 0;
             est_sum += (long long)est;
         }
+        if (sg.cap == 0) continue;
         int tot;
         const int ex = warp_excl_scan(nit, tot);
         unsigned long long base = 0;
@@ -446,17 +430,23 @@ __global__ void __launch_bounds__(256) k_seg_count(DiscArgs a, SegArgs sg) {
         atomicAdd((unsigned long long *)(a.ctr + C_SEG_EST), (unsigned long long)est_sum);
 }
 
-// The chunk's mode: segmented when its estimated deposits reach min_est and
-// its items fit the item buffers (else the per-disc kernels deposit in FP64).
+// The chunk's mode.  From min_est estimated deposits on it is rendered by
+// tiles where the pair list holds its pairs, else in segments where the item
+// buffers hold its items, else (and below min_est) by the per-disc kernels
+// with FP64 deposits.
 __global__ void k_seg_decide(DiscArgs a, SegArgs sg) {
-    const long long items = a.ctr[C_SEG_ITEMS], est = a.ctr[C_SEG_EST];
-    const int mode = (items > 0 && items <= sg.cap && est >= sg.min_est) ? 1 : 0;
+    int mode = 0;
+    if (a.ctr[C_SEG_EST] >= sg.min_est && a.ctr[C_ADD_BLOCK] > 0) {
+        const long long items = a.ctr[C_SEG_ITEMS];
+        if (sg.pair_cap > 0 && a.ctr[C_TILE_BOUND] <= sg.pair_cap) mode = 2;
+        else if (items > 0 && items <= sg.cap) mode = 1;
+    }
     sg.ctl[0] = mode;
     a.ctr[C_SEG_MODE] = mode;
 }
 
 __global__ void __launch_bounds__(256) k_seg_fill(DiscArgs a, SegArgs sg) {
-    if (sg.ctl[0] == 0) return;
+    if (sg.ctl[0] != 1) return;
     const long long nblk = a.ctr[C_ADD_BLOCK];
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nblk; q += stride) {
@@ -478,7 +468,7 @@ __device__ inline int seg_class(const DiscArgs &a, const SegArgs &sg, long long 
 
 // Items and pixels per class (sg.cls[0 .. kClasses), sg.cls_px).
 __global__ void __launch_bounds__(256) k_seg_class(DiscArgs a, SegArgs sg) {
-    if (sg.ctl[0] == 0) return;
+    if (sg.ctl[0] != 1) return;
     __shared__ int hist[kClasses];
     __shared__ unsigned long long px[kClasses];
     for (int i = threadIdx.x; i < kClasses; i += blockDim.x) {
@@ -503,7 +493,7 @@ __global__ void __launch_bounds__(256) k_seg_class(DiscArgs a, SegArgs sg) {
 // Exclusive scan of the class histogram into the classes' first slots
 // (sg.cls[kClasses .. 2 kClasses)); one block of kClasses threads.
 __global__ void __launch_bounds__(kClasses) k_seg_cscan(SegArgs sg) {
-    if (sg.ctl[0] == 0) return;
+    if (sg.ctl[0] != 1) return;
     int total;
     const int v = sg.cls[threadIdx.x];
     const int ex = warp_excl_scan(v, total);
@@ -517,7 +507,7 @@ __global__ void __launch_bounds__(kClasses) k_seg_cscan(SegArgs sg) {
 
 // Each disc's items into its class's range of the sorted list.
 __global__ void __launch_bounds__(256) k_seg_sort(DiscArgs a, SegArgs sg) {
-    if (sg.ctl[0] == 0) return;
+    if (sg.ctl[0] != 1) return;
     const long long nblk = a.ctr[C_ADD_BLOCK];
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nblk; q += stride) {
@@ -529,7 +519,7 @@ __global__ void __launch_bounds__(256) k_seg_sort(DiscArgs a, SegArgs sg) {
 
 // The segment plan (plan_segments in seg_plan.h), one thread.
 __global__ void k_seg_plan(SegArgs sg) {
-    if (sg.ctl[0] == 0) return;
+    if (sg.ctl[0] != 1) return;
     sg.ctl[1] = plan_segments(sg.cls, sg.cls + kClasses, sg.cls_px, sg.budget, sg.spans);
 }
 
@@ -537,7 +527,7 @@ __global__ void k_seg_plan(SegArgs sg) {
 // npix is a multiple of 4); returns at once when the plan has no segment seg.
 __global__ void __launch_bounds__(256) k_seg_flush(const int *ctl, int seg, float *plane, double *acc,
                                                    long long npix4) {
-    if (ctl[0] == 0 || seg >= ctl[1]) return;
+    if (ctl[0] != 1 || seg >= ctl[1]) return;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < npix4; i += stride) {
         const float4 v = reinterpret_cast<float4 *>(plane)[i];
@@ -598,8 +588,10 @@ cudaError_t launch_seg_count(const DiscArgs &a, const SegArgs &sg, int block_thr
                              cudaStream_t s) {
     if (block_threads == 256) k_seg_count<256><<<num_sms * 8, 256, 0, s>>>(a, sg);
     else k_seg_count<128><<<num_sms * 8, 256, 0, s>>>(a, sg);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_seg_decide(const DiscArgs &a, const SegArgs &sg, cudaStream_t s) {
     k_seg_decide<<<1, 1, 0, s>>>(a, sg);
     return cudaGetLastError();
 }

@@ -41,7 +41,16 @@ enum Ctr {
     C_SEG_ITEMS,       // work items of the chunk's block-class discs
     C_SEG_EST,         // their estimated pixels (cap areas)
     C_SEG_NEXT_NORM,   // items claimed by pass 1
-    C_SEG_MODE,        // 1: the chunk took the segmented render
+    C_SEG_MODE,        // the chunk's render: 0 per-disc kernels, 1 segments, 2 tiles
+    // tiled render (disc_tile.cu)
+    C_TILE_BOUND,      // (disc, tile) pairs, counted before the mode is known
+    C_TILE_PAIRS,      // the pairs of the three lists
+    C_TILE_PAIRS_LAST = C_TILE_PAIRS + 2,
+    C_TILE_NEXT, C_GEN, C_GEN_NEXT,     // discs claimed; giant discs, parts of them claimed
+    C_TILE_CURSOR,     // pair list slots handed out
+    C_UNITS, C_UNEXT = C_UNITS + 3,     // work units of the three lists, and claims
+    C_UNEXT_LAST = C_UNEXT + 2,
+    C_OCT_MAX,         // largest biased FP32 exponent of F
     C_COUNT
 };
 constexpr int kCtrChunkFirst = C_ADD_DISC;
@@ -119,12 +128,13 @@ struct DiscArgs {
 struct SegArgs {
     int2 *items;              // (queue slot, item index within its disc), queue order
     int2 *sorted;             // the same items in ascending octave of the disc's F
-    long long cap;            // capacity of items and sorted
+    long long cap;            // capacity of items and sorted (0: no segmented render)
+    long long pair_cap;       // capacity of the tiled render's pair list (0: none)
     int *cls;                 // [2 kClasses]: items per octave, then each octave's first slot
     long long *cls_px;        // [kClasses]: pixels (deposits) per octave
     unsigned long long *seg_next;   // [kSegSlots]: items claimed by each segment
     SegSpan *spans;           // [kSegSlots]: the segment plan
-    int *ctl;                 // [0] mode (1 segmented, 0 per-disc kernels), [1] segments
+    int *ctl;                 // [0] mode (0 per-disc kernels, 1 segmented, 2 tiled), [1] segments
     long long min_est;        // estimated deposits from which the chunk is segmented
     long long budget;         // deposits per segment before the plan splits an octave
     long long *disc_first;    // per block-class disc: its first item
@@ -133,6 +143,48 @@ struct SegArgs {
     long long *disc_px;       //   its pixel count (pass 1)
     float *plane;             // FP32 deposit plane, npix floats, zero between segments
 };
+
+// Tiled render of the block-class discs (disc_tile.cu): a tile is kTileR rings
+// by kTileW in-ring pixel indices, a unit up to kUnitMax discs of its list
+// (fewer while the chunk has less than kUnitTarget units of more than kUnitMin).
+constexpr int kTileR = 32, kTileW = 64;
+constexpr int kUnitMin = 32, kUnitMax = 512, kUnitTarget = 16384;
+constexpr int kTileClasses = 64;
+
+struct TileUnit {
+    long long start;   // of its part of the pair list
+    int len, tile;
+};
+
+// What the tiled render reads of one disc (64 bytes of the 160 of its header;
+// a pair of disc and tile reads it once).
+struct alignas(16) TileHdr {
+    float t0h, t0l;         // theta0 as a two-float
+    float hR, sth0;         // hav(R), sin(theta0)
+    float nK;
+    float F, Fn, p;         // flux / S lies a share p of the way from F to its neighbour Fn
+    float ph, pl;           // phi0 / 2 pi as a two-float
+    int r_first, r_last, irmin, irmax;   // as DiscHdr
+    int q, flags;           // queue slot; kind and flags (disc_tile.cu)
+};
+static_assert(sizeof(TileHdr) == 64, "four 16-byte words");
+
+struct TileArgs {
+    TileHdr *hdr;             // per block-class disc
+    const int *ctl;           // SegArgs::ctl: 2 when the chunk is rendered by tiles
+    int nstrips, ncol;        // tiles of the map: strips of kTileR rings x columns
+    unsigned *list;           // the pairs' discs, tile by tile
+    unsigned *hist;           // [3 tiles][kTileClasses]: pairs per octave, then list slots (a third per list)
+    long long *base;          // [3 tiles]: each tile's first list slot
+    TileUnit *units;          // [3][unit_cap]
+    long long unit_cap;
+    double *disc_S;           // per block-class disc, as SegArgs
+    long long *disc_px;
+    int *gen;                 // queue slots of the giant discs (C_GEN of them)
+};
+
+inline int tile_strips(int nside) { return (4 * nside - 1 + kTileR - 1) / kTileR; }
+inline int tile_cols(int nside) { return (4 * nside + kTileW - 1) / kTileW; }
 
 // prep.cu
 cudaError_t launch_prep(const PrepArgs &a, cudaStream_t s);
@@ -167,11 +219,18 @@ cudaError_t launch_disc_comp_warp(const DiscArgs &a, int num_sms, cudaStream_t s
 // picks the block shape.
 cudaError_t launch_seg_count(const DiscArgs &a, const SegArgs &sg, int block_threads, int num_sms,
                              cudaStream_t s);
+cudaError_t launch_seg_decide(const DiscArgs &a, const SegArgs &sg, cudaStream_t s);
 cudaError_t launch_seg_norm(const DiscArgs &a, const SegArgs &sg, int block_threads, int num_sms,
                             int blocks_per_sm, cudaStream_t s);
 cudaError_t launch_seg_sort(const DiscArgs &a, const SegArgs &sg, int num_sms, cudaStream_t s);
 cudaError_t launch_seg_deposits(const DiscArgs &a, const SegArgs &sg, int block_threads, int num_sms,
                                 int blocks_per_sm, int npix, cudaStream_t s);
+// disc_tile.cu, in stream order, each returning at once unless the chunk's
+// mode is 2: the tile headers and (total) the pair count, before the mode is
+// decided; the weight sums; F, the pair list and the deposits.
+cudaError_t launch_tile_hdr(const DiscArgs &a, const TileArgs &tg, bool total, int num_sms, cudaStream_t s);
+cudaError_t launch_tile_norm(const DiscArgs &a, const TileArgs &tg, int num_sms, cudaStream_t s);
+cudaError_t launch_tile_deposits(const DiscArgs &a, const TileArgs &tg, int num_sms, cudaStream_t s);
 // disc_comp.cu: the compensated block kernel alone (headers built)
 cudaError_t launch_disc_comp_block(const DiscArgs &a, int num_sms, int blocks_per_sm, int block_threads,
                                    cudaStream_t s);

@@ -107,9 +107,10 @@ typedef struct {
     int64_t launches;      /* kernels launched for the last map (all chunks) */
     double pass1_ms;       /* compensated form, block class of the last chunk: from the
                               disc kernels' start to the end of the weight sums (headers,
-                              work items, pass 1) */
-    double pass2_ms;       /* the item sort, the deposit segments and their flushes
-                              (both 0 when the chunk deposited in FP64) */
+                              counts, pass 1) */
+    double pass2_ms;       /* the pair list and the tiles' deposits, or the item sort,
+                              the deposit segments and their flushes (both 0 when the
+                              chunk deposited in FP64) */
 } dmann_stats;
 
 /* Tunables (set by the annmap autotuner; zero fields keep the current
@@ -127,10 +128,11 @@ typedef struct {
                                   block shape (192, 384, 640) */
     int32_t seg_min_deposits_log2;  /* compensated form: a chunk whose block-
                                   class discs are estimated to make at least
-                                  2^this many deposits takes the segmented
-                                  render (FP32 deposits flushed into the FP64
-                                  plane per segment, 128 or 256 threads);
-                                  smaller chunks deposit in FP64.  1 .. 62 */
+                                  2^this many deposits is rendered by map
+                                  tiles (or in segments where the tiles' disc
+                                  lists would not fit): short FP32 sums added
+                                  into the FP64 plane; smaller chunks deposit
+                                  in FP64.  1 .. 62 */
     int32_t reserved[2];
 } dmann_tuning;
 
