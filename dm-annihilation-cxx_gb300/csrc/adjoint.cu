@@ -19,8 +19,8 @@
 //   dL/dR[j][a] = K (D V)_a u_j / d  (through n only).
 // The pixel sets are held fixed (the derivative of the map where disc
 // membership does not change); the single-pixel case has V = T = 0.
-// The weights are recomputed (two passes over the disc: S and sum g w, then
-// V and T), not stored.  Compiled with -fmad=false like the plain form, so
+// Two passes over the disc: S and sum g w, then V and T, with the weights of
+// the first kept as far as the group's scratch reaches.  Compiled with -fmad=false like the plain form, so
 // the weights and S are bit for bit those of the plain forward kernels.
 // With precision DMANN_COMP_F32 the disc particles go to the compensated
 // form's kernels instead (disc_comp.cu), with FP32 weights.
@@ -43,10 +43,13 @@ struct AdjSmem {
 // Gradient of one disc particle with a group of G threads.  The group's
 // rank 0 adds the observer terms into acc.
 template <int G, int RCH>
-__device__ inline void adjoint_particle(const AdjArgs &a, AdjSmem<RCH> &sm, int pidx,
+__device__ inline void adjoint_particle(const AdjArgs &a, AdjSmem<RCH> &sm, int pidx, long long group,
                                         double acc[12]) {
     using Grp = Group<G>;
     const DiscArgs &da = a.d;
+    // (weight, angular distance) of the pixels, kept for pass 2
+    const long long kept = da.scratch ? da.scratch_len : 0;
+    double2 *const wbuf = reinterpret_cast<double2 *>(da.scratch) + group * da.scratch_len;
     const int r = Grp::rank();
     if (r == 0) {
         disc_setup(da.g, da.theta[pidx], da.phi[pidx], da.ar[pidx], da.flux[pidx], da.cpix[pidx],
@@ -68,13 +71,17 @@ __device__ inline void adjoint_particle(const AdjArgs &a, AdjSmem<RCH> &sm, int 
         const int nr = min(RCH, r_last - r0 + 1);
         build_chunk<PlainForm, G, RCH>(da, sm.g, r0, nr);
         const int ct = (int)sm.g.chunk_total;
-        total += ct;
-        pixel_walk<PlainForm, G, RCH>(sm.g, nr, ct, [&](const PlainForm::SegReg &sr, int j, int pix) {
-            (void)j;
-            const double w = PlainForm::weight(ext, sr, pix);
+        pixel_walk<PlainForm, G, RCH>(sm.g, nr, ct, [&](const PlainForm::SegReg &sr, int f, int pix) {
+            double px, py, pz;
+            PlainForm::pixel_vec(ext, sr, pix, px, py, pz);
+            const double dot = px * ext.vx + py * ext.vy + pz * ext.vz;
+            const double alpha = acos(fmin(1.0, fmax(-1.0, dot)));
+            const double w = PlainForm::weight_at(ext, alpha);
             s1[0] += w;
             s1[1] += gmap[pix] * w;
+            if (total + f < kept) wbuf[total + f] = make_double2(w, alpha);
         });
+        total += ct;
         Grp::sync();
     }
     group_sum<G, 2>(s1, sm.red);
@@ -94,31 +101,37 @@ __device__ inline void adjoint_particle(const AdjArgs &a, AdjSmem<RCH> &sm, int 
     // pass 2: V and T with q = (G - Gm) w (the staged chunk is reused when
     // there is only one)
     double s2[4] = {0.0, 0.0, 0.0, 0.0};
+    long long done = 0;
     for (int c = 0; c < nchunk; c++) {
         const int r0 = r_first + c * RCH;
         const int nr = min(RCH, r_last - r0 + 1);
         if (nchunk > 1) build_chunk<PlainForm, G, RCH>(da, sm.g, r0, nr);
         const int ct = (int)sm.g.chunk_total;
-        pixel_walk<PlainForm, G, RCH>(sm.g, nr, ct, [&](const PlainForm::SegReg &sr, int j, int pix) {
-            (void)j;
+        pixel_walk<PlainForm, G, RCH>(sm.g, nr, ct, [&](const PlainForm::SegReg &sr, int f, int pix) {
             double px, py, pz;
             PlainForm::pixel_vec(ext, sr, pix, px, py, pz);
             const double dot = px * ext.vx + py * ext.vy + pz * ext.vz;
             const double dc = fmin(1.0, fmax(-1.0, dot));
-            const double alpha = acos(dc);
-            double d2 = alpha / ext.ar;
-            d2 = d2 * d2;
-            const double w = exp(-0.5 * d2 / 0.333);
+            double w, alpha;
+            if (done + f < kept) {
+                const double2 k = wbuf[done + f];
+                w = k.x;
+                alpha = k.y;
+            } else {
+                alpha = acos(dc);
+                w = PlainForm::weight_at(ext, alpha);
+            }
             const double q = (gmap[pix] - Gm) * w;
             // tangent of the great circle from n towards the pixel, length sin(alpha)
             const double ex = px - dc * ext.vx, ey = py - dc * ext.vy, ez = pz - dc * ext.vz;
             const double sa = sqrt(ex * ex + ey * ey + ez * ez);
-            const double f = sa > 0.0 ? q * alpha / sa : 0.0;
-            s2[0] += f * ex;
-            s2[1] += f * ey;
-            s2[2] += f * ez;
+            const double t = sa > 0.0 ? q * alpha / sa : 0.0;
+            s2[0] += t * ex;
+            s2[1] += t * ey;
+            s2[2] += t * ez;
             s2[3] += q * alpha * alpha;
         });
+        done += ct;
         Grp::sync();
     }
     group_sum<G, 4>(s2, sm.red);
@@ -143,7 +156,7 @@ __global__ void __launch_bounds__(BT, 1) k_adj_block(AdjArgs a) {
         const int q = s_q;
         __syncthreads();
         if (q >= nblk) break;
-        adjoint_particle<BT, RCH>(a, sm, a.d.queue[q], acc);
+        adjoint_particle<BT, RCH>(a, sm, a.d.queue[q], blockIdx.x, acc);
     }
     if (threadIdx.x == 0) flush_acc(a.oacc, acc);
 }
@@ -157,7 +170,7 @@ __global__ void __launch_bounds__(WPB * 32) k_adj_warp(AdjArgs a) {
     const int w = threadIdx.x >> 5;
     const long long gw = (long long)blockIdx.x * WPB + w;
     const long long nw = (long long)gridDim.x * WPB;
-    for (long long q = nblk + gw; q < ndisc; q += nw) adjoint_particle<32, RCH>(a, sm[w], a.d.queue[q], acc);
+    for (long long q = nblk + gw; q < ndisc; q += nw) adjoint_particle<32, RCH>(a, sm[w], a.d.queue[q], gw, acc);
     if ((threadIdx.x & 31) == 0) flush_acc(a.oacc, acc);
 }
 
@@ -226,12 +239,14 @@ cudaError_t launch_adjoint(const DiscArgs &d, const Particles &p, const signed c
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adj_block<kBT, kRCH>, kBT, 0);
     if (e != cudaSuccess) return e;
     if (occ < 1) occ = 1;
+    a.d.scratch_len = d.scratch_total / 2 / (num_sms * occ);
     k_adj_block<kBT, kRCH><<<num_sms * occ, kBT, 0, s>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int occw = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occw, k_adj_warp<kWPB, kRCHW>, kWPB * 32, 0);
     if (e != cudaSuccess) return e;
     if (occw < 1) occw = 1;
+    a.d.scratch_len = d.scratch_total / 2 / (num_sms * occw * kWPB);
     k_adj_warp<kWPB, kRCHW><<<num_sms * occw, kWPB * 32, 0, s>>>(a);
     return cudaGetLastError();
 }

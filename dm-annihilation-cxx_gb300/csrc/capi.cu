@@ -31,6 +31,7 @@ struct RingTables {
     double *z = nullptr, *st = nullptr, *theta = nullptr, *step = nullptr;
     float *st32 = nullptr, *step32 = nullptr;
     float2 *th2 = nullptr;
+    double2 *trig_belt = nullptr, *trig_cap = nullptr;   // the plain form's, built on first use
 };
 
 }  // namespace
@@ -48,6 +49,7 @@ struct Work {
     bool plane_clean = false;   // plane32 is all zero (every segment's flush leaves it so)
     // tiled render (disc_tile.cu): the pair list, its histogram and ranges,
     // the work units, the general discs
+    DevBuf scratch;           // plain form: the weights of the discs in work
     DevBuf tile_hdr, tile_list, tile_hist, tile_base, tile_units, tile_gen;
 };
 
@@ -176,6 +178,46 @@ bool ensure_opt(DevBuf &b, size_t bytes) {
         b.p = nullptr;
     }
     return false;
+}
+
+// The plain form's scratch (2^25 doubles: 55,000 pixels' weights for each of
+// the 608 blocks of the block kernel; less for small maps) and, per Nside, its
+// (sin, cos) tables.  All optional: what is missing is computed again.
+void reserve_plain(dmann_ctx *ctx, int nside) {
+    const size_t npix = 12 * (size_t)nside * (size_t)nside;
+    ensure_opt(ctx->w->scratch, 8 * std::min((size_t)1 << 25, 32768 * npix));
+    auto it = ctx->rings.find(nside);
+    if (it == ctx->rings.end() || it->second.trig_belt) return;
+    RingTables &t = it->second;
+    const size_t cap = 2 * (size_t)nside * (nside - 1);
+    if (cudaMalloc(&t.trig_belt, sizeof(double2) * 8 * nside) != cudaSuccess) {
+        cudaGetLastError();
+        t.trig_belt = nullptr;
+        return;
+    }
+    // a cap's table up to Nside 1448 (64 MB)
+    if (cap > 0 && sizeof(double2) * cap <= ((size_t)64 << 20) &&
+        cudaMalloc(&t.trig_cap, sizeof(double2) * cap) != cudaSuccess) {
+        cudaGetLastError();
+        t.trig_cap = nullptr;
+    }
+    // the tables outlive this map and its stream: complete before any use
+    if (launch_trig(nside, (double)(nside << 1) * (4.0 / (double)npix), t.trig_belt, t.trig_cap, ctx->stream) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        cudaFree(t.trig_belt);
+        if (t.trig_cap) cudaFree(t.trig_cap);
+        t.trig_belt = t.trig_cap = nullptr;
+    }
+}
+
+void plain_args(const dmann_ctx *ctx, int nside, DiscArgs &da) {
+    da.scratch = (double *)ctx->w->scratch.p;
+    da.scratch_total = (long long)(ctx->w->scratch.bytes / 8);
+    auto it = ctx->rings.find(nside);
+    if (it == ctx->rings.end()) return;
+    da.trig_belt = it->second.trig_belt;
+    da.trig_cap = it->second.trig_cap;
 }
 
 CompHdr *headers_for(const dmann_ctx *ctx, size_t n) {
@@ -378,7 +420,7 @@ void dmann_destroy(dmann_ctx *ctx) {
         DevBuf *wb[] = {&wk.theta, &wk.phi, &wk.ar, &wk.flux, &wk.cpix, &wk.key, &wk.queue, &wk.hist,
                         &wk.ctr, &wk.fsum, &wk.acc, &wk.chdr, &wk.seg_items, &wk.seg_sorted,
                         &wk.seg_cls, &wk.seg_first, &wk.seg_nit, &wk.seg_S, &wk.seg_px, &wk.plane32,
-                        &wk.tile_hdr, &wk.tile_list, &wk.tile_hist, &wk.tile_base, &wk.tile_units, &wk.tile_gen};
+                        &wk.scratch, &wk.tile_hdr, &wk.tile_list, &wk.tile_hist, &wk.tile_base, &wk.tile_units, &wk.tile_gen};
         for (DevBuf *b : wb)
             if (b->p) cudaFree(b->p);
     }
@@ -396,6 +438,8 @@ void dmann_destroy(dmann_ctx *ctx) {
         cudaFree(kv.second.st32);
         cudaFree(kv.second.step32);
         cudaFree(kv.second.th2);
+        if (kv.second.trig_belt) cudaFree(kv.second.trig_belt);
+        if (kv.second.trig_cap) cudaFree(kv.second.trig_cap);
     }
     if (ctx->h_ctr) cudaFreeHost(ctx->h_ctr);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -885,6 +929,7 @@ dmann_status dmann_map_add_v(dmann_ctx *ctx, const float *x, const float *y, con
         (st = ensure(ctx, ctx->w->queue, 4 * N)))
         return st;
     if (ctx->precision == DMANN_COMP_F32) reserve_headers(ctx, N);
+    else reserve_plain(ctx, ctx->g.nside);
     // inputs: device pointers are used in place, host arrays are copied
     const float *src[7] = {x, y, z, m, rho, h, law_needs_sigmav(ctx->flux_model) ? sigmav : nullptr};
     const float *dev[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -946,6 +991,7 @@ dmann_status dmann_map_add_v(dmann_ctx *ctx, const float *x, const float *y, con
     if (ctx->precision == DMANN_COMP_F32) da.chdr = headers_for(ctx, N);
     CK(cudaEventRecord(ctx->evd0, s));
     if (ctx->precision == DMANN_PLAIN_F64) {
+        plain_args(ctx, ctx->g.nside, da);
         CK(launch_disc_plain(da, ctx->num_sms, tu.blocks_per_sm, s, ctx->evdm));
         ctx->launches += 5;   // prep, scan, scatter, disc block, disc warp
     } else {
@@ -1086,6 +1132,7 @@ dmann_status issue_observer(dmann_ctx *ctx, const float *const dev[6], int n, in
         da.ctr = pa.ctr;
         da.acc = acc;
         if (precision == DMANN_PLAIN_F64) {
+            plain_args(ctx, nside, da);
             CK(launch_disc_plain(da, ctx->num_sms, tu.blocks_per_sm, s, nullptr));
         } else {
             da.chdr = headers_for(ctx, (size_t)n);
@@ -1176,6 +1223,12 @@ dmann_status dmann_render_batch(dmann_ctx *ctx, const float *x, const float *y, 
     std::vector<RingTables> rts(n_obs);
     for (int k = 0; k < n_obs; k++)
         if ((st = ring_tables(ctx, nside[k], rts[k])) != DMANN_OK) return st;
+    if (precision == DMANN_PLAIN_F64)
+        for (int L = 0; L < lanes; L++) {
+            ctx->w = &ctx->work[L];
+            for (int k = 0; k < n_obs; k++) reserve_plain(ctx, nside[k]);
+            ctx->w = &ctx->work[0];
+        }
     const float *src[6] = {x, y, z, m, rho, h};
     const float *dev[6];
     for (int k = 0; k < 6; k++) {
@@ -1387,6 +1440,8 @@ dmann_status dmann_adjoint_v(dmann_ctx *ctx, const float *x, const float *y, con
     if (precision == DMANN_COMP_F32) {
         if ((st = ensure(ctx, ctx->w->acc, 4 * P)) != DMANN_OK) return st;
         reserve_headers(ctx, n1);
+    } else {
+        reserve_plain(ctx, nside);
     }
     const float *src[7] = {x, y, z, m, rho, h, law_needs_sigmav(ctx->flux_model) ? sigmav : nullptr};
     const float *dev[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -1455,6 +1510,7 @@ dmann_status dmann_adjoint_v(dmann_ctx *ctx, const float *x, const float *y, con
     da.ctr = pa.ctr;
     da.acc = pa.acc;
     if (precision == DMANN_COMP_F32) da.chdr = headers_for(ctx, n1);
+    else plain_args(ctx, nside, da);
     CK(cudaEventRecord(ctx->evd0, s));
     CK(launch_adjoint(da, pa.p, pa.out.cls, dgmap, (float *)ctx->w->acc.p, dgrad, (double *)ctx->oacc.p,
                       precision, ctx->num_sms, s, core ? (const double *)ctx->corr.p : nullptr,

@@ -14,8 +14,8 @@
 // group then walks the chunk's pixels as one flattened index space, each
 // warp taking a contiguous stretch with lanes on consecutive pixels, so
 // lanes of a warp touch consecutive map addresses.  Pass 1 sums the weights
-// (the per-particle normalisation); pass 2 recomputes them and deposits
-// w * flux / norm.  A disc with fewer than 2 pixels puts its whole flux into
+// (the per-particle normalisation) and keeps them; pass 2 deposits w * flux /
+// norm.  A disc with fewer than 2 pixels puts its whole flux into
 // the centre pixel (genmap.cpp:125-128).
 #pragma once
 #include "kernels.cuh"
@@ -111,7 +111,8 @@ __device__ inline int find_seg(const Seg *seg, int n, int f) {
     return lo;
 }
 
-// Walks the chunk's flattened pixels; `body(seg_cache, j, pix)` per pixel.
+// Walks the chunk's flattened pixels; `body(seg_cache, f, pix)` per pixel, f its
+// index in the chunk (a thread meets the same f whenever it walks the chunk).
 template <class Form, int G, int RCH, class Body>
 __device__ inline void pixel_walk(const GroupSmem<Form, RCH> &sm, int n, int total, Body body) {
     using Grp = Group<G>;
@@ -135,7 +136,7 @@ __device__ inline void pixel_walk(const GroupSmem<Form, RCH> &sm, int n, int tot
         int k = cur.lo + j;
         k += (k < 0) ? cur.nr : 0;
         k -= (k >= cur.nr) ? cur.nr : 0;
-        body(cur, j, cur.start + k);
+        body(cur, f, cur.start + k);
         f += 32;
         if (f >= seg_end && f < f1) {
             do {
@@ -149,8 +150,10 @@ __device__ inline void pixel_walk(const GroupSmem<Form, RCH> &sm, int n, int tot
 }
 
 template <class Form, int G, int RCH>
-__device__ inline void render_particle(const DiscArgs &a, GroupSmem<Form, RCH> &sm, int pidx) {
+__device__ inline void render_particle(const DiscArgs &a, GroupSmem<Form, RCH> &sm, int pidx, long long group) {
     using Grp = Group<G>;
+    const long long kept = a.scratch ? a.scratch_len : 0;   // pixels whose weights are kept
+    double *const wbuf = a.scratch + group * a.scratch_len;
     const int r = Grp::rank();
     if (r == 0) {
         disc_setup(a.g, a.theta[pidx], a.phi[pidx], a.ar[pidx], a.flux[pidx], a.cpix[pidx], pidx,
@@ -163,21 +166,24 @@ __device__ inline void render_particle(const DiscArgs &a, GroupSmem<Form, RCH> &
     const int nring = r_last - r_first + 1;
     const int nchunk = nring > 0 ? (nring + RCH - 1) / RCH : 0;
 
-    // pass 1: normalisation
-    typename Form::NormAcc nacc;
+    // pass 1: normalisation.  The weights (about 75 FP64 operations each, on a
+    // pipe at 1/64 of the FP32 rate) are kept for pass 2 as far as the group's
+    // scratch reaches; a thread reads back only what it wrote.
+    double part = 0.0;
     long long total = 0;
     for (int c = 0; c < nchunk; c++) {
         const int r0 = r_first + c * RCH;
         const int n = min(RCH, r_last - r0 + 1);
         build_chunk<Form, G, RCH>(a, sm, r0, n);
         const int ct = (int)sm.chunk_total;
-        total += ct;
-        pixel_walk<Form, G, RCH>(sm, n, ct, [&](const typename Form::SegReg &sr, int j, int pix) {
-            Form::norm_add(ext, sr, j, pix, nacc);
+        pixel_walk<Form, G, RCH>(sm, n, ct, [&](const typename Form::SegReg &sr, int f, int pix) {
+            const double w = Form::weight(ext, sr, pix);
+            part += w;
+            if (total + f < kept) wbuf[total + f] = w;
         });
+        total += ct;
         Grp::sync();
     }
-    double part = Form::norm_value(nacc);
     part = warp_sum(part);
     double S = part;
     if (G > 32) {
@@ -197,17 +203,20 @@ __device__ inline void render_particle(const DiscArgs &a, GroupSmem<Form, RCH> &
     }
     if (r == 0) atomicAdd((unsigned long long *)(a.ctr + C_DEPOSITS), (unsigned long long)total);
     typename Form::Dep dep;
-    Form::deposit_setup(a, sm.hdr, ext, S, dep);
+    Form::deposit_setup(sm.hdr, S, dep);
 
     // pass 2: deposits (the staged chunk is reused when there is only one)
+    long long done = 0;
     for (int c = 0; c < nchunk; c++) {
         const int r0 = r_first + c * RCH;
         const int n = min(RCH, r_last - r0 + 1);
         if (nchunk > 1) build_chunk<Form, G, RCH>(a, sm, r0, n);
         const int ct = (int)sm.chunk_total;
-        pixel_walk<Form, G, RCH>(sm, n, ct, [&](const typename Form::SegReg &sr, int j, int pix) {
-            Form::deposit(a, ext, dep, sr, j, pix);
+        pixel_walk<Form, G, RCH>(sm, n, ct, [&](const typename Form::SegReg &sr, int f, int pix) {
+            const double w = done + f < kept ? wbuf[done + f] : Form::weight(ext, sr, pix);
+            Form::deposit(a, dep, w, pix);
         });
+        done += ct;
         Grp::sync();
     }
 }
@@ -228,7 +237,7 @@ __global__ void __launch_bounds__(BT, Form::kMinBlocks) k_disc_block(DiscArgs a)
         const int q = s_q;
         __syncthreads();
         if (q >= nblk) break;
-        render_particle<Form, BT, RCH>(a, sm, a.queue[q]);
+        render_particle<Form, BT, RCH>(a, sm, a.queue[q], blockIdx.x);
     }
 }
 
@@ -242,7 +251,7 @@ __global__ void __launch_bounds__(WPB * 32) k_disc_warp(DiscArgs a) {
     const long long gw = (long long)blockIdx.x * WPB + w;
     const long long nw = (long long)gridDim.x * WPB;
     for (long long q = nblk + gw; q < ndisc; q += nw) {
-        render_particle<Form, 32, RCH>(a, sm[w], a.queue[q]);
+        render_particle<Form, 32, RCH>(a, sm[w], a.queue[q], gw);
     }
 }
 

@@ -120,6 +120,13 @@ struct DiscArgs {
     // compensated block kernel: returns at once when *block_skip != 0 (the
     // segmented render took the chunk's block class); null = never
     const int *block_skip = nullptr;
+    // plain form: FP64 scratch for the weights of the discs in work (doubles;
+    // scratch_len per group of threads, set by the launch), and (sin, cos) of
+    // every pixel azimuth: two rings of the belt (4 nside each, shifted and not)
+    // and the rings of a cap.  Each optional (null: recomputed).
+    double *scratch = nullptr;
+    long long scratch_total = 0, scratch_len = 0;
+    const double2 *trig_belt = nullptr, *trig_cap = nullptr;
 };
 
 
@@ -199,6 +206,9 @@ cudaError_t launch_halo_core(const HaloGrid &g, const Particles &p, double *corr
 // disc_plain.cu / disc_comp.cu
 // Launch the block-per-particle kernel, record `mid` (if not null), then the
 // warp-per-particle kernel.
+// (sin, cos) tables of the plain form: 8 nside of the belt; 2 nside (nside - 1)
+// of a cap (cap may be null)
+cudaError_t launch_trig(int nside, double fact1, double2 *belt, double2 *cap, cudaStream_t s);
 cudaError_t launch_disc_plain(const DiscArgs &a, int num_sms, int blocks_per_sm, cudaStream_t s,
                               cudaEvent_t mid);
 // block_threads: 128, 256 or 512 (the compensated block kernel's shape;

@@ -10,6 +10,26 @@
 
 namespace dmann {
 
+// a / b, correctly rounded, from r = RN(1 / b): the quotient a r is within
+// two ulp, one correction makes it faithful, and by Markstein's theorem (IBM
+// J. Res. Dev. 34, 1990) a second one rounds it correctly.  Five FP64
+// operations where the general division takes about twice as many; the
+// divisors here serve a whole disc.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+    double q = __dmul_rn(a, r);
+    q = __fma_rn(__fma_rn(-q, b, a), r, q);
+    return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
+
+// The azimuth of pixel k (from 0) of a cap ring (ipole rings from its pole)
+// and of an equatorial ring (pf: 1/2 or 1), as pix2vec forms them.
+__device__ __forceinline__ double cap_phi(int k, int ipole) {
+    return ((double)(k + 1) - 0.5) * kHalfPi / (double)ipole;
+}
+__device__ __forceinline__ double belt_phi(int k, double pf, double fact1) {
+    return ((double)(k + 1) - pf) * kPi * 0.75 * fact1;
+}
+
 struct PlainForm {
     static constexpr bool kFastChord = false;  // the exact FP64 chord test
     static constexpr int kMinBlocks = 1;
@@ -17,20 +37,19 @@ struct PlainForm {
         int start, nr, lo, off;
         double z, st, pf;
         int cap, ipole;
+        const double2 *trig;   // (sin, cos) of the ring's pixels, or null
     };
     struct SegReg {
         int start, nr, lo;
         double z, st, pf;
         int cap, ipole;
+        const double2 *trig;
     };
     struct Ext {
-        double vx, vy, vz, ar, fact1;
-    };
-    struct NormAcc {
-        double s = 0.0;
+        double vx, vy, vz, ar, fact1, inv_ar;
     };
     struct Dep {
-        double S, flux;
+        double S, inv_S, flux;
     };
 
     // anglefuncs.cpp:55-71 ang2vec, from the un-normalised phi of calc_angles
@@ -41,6 +60,7 @@ struct PlainForm {
         e.vy = sz * sin(phi_raw);
         e.vz = cos(d.theta0);
         e.ar = d.ar;
+        e.inv_ar = __ddiv_rn(1.0, d.ar);
         e.fact1 = a.g.fact1;
     }
 
@@ -58,6 +78,8 @@ struct PlainForm {
         s.cap = (ring < ns) || (ring > 3 * ns);
         s.ipole = (ring < ns) ? ring : 4 * ns - ring;
         s.pf = ((ring + ns) & 1) ? 1.0 : 0.5;
+        if (s.cap) s.trig = a.trig_cap ? a.trig_cap + 2LL * s.ipole * (s.ipole - 1) : nullptr;
+        else s.trig = a.trig_belt ? a.trig_belt + (s.pf == 1.0 ? 4 * ns : 0) : nullptr;
     }
 
     __device__ static void load_seg(const Seg &s, SegReg &r) {
@@ -69,52 +91,47 @@ struct PlainForm {
         r.pf = s.pf;
         r.cap = s.cap;
         r.ipole = s.ipole;
+        r.trig = s.trig;
     }
 
     // pix2vec of a pixel of the segment's ring, as the oracle restates it
     __device__ static void pixel_vec(const Ext &e, const SegReg &sr, int pix, double &px,
                                      double &py, double &pz) {
         const int k = pix - sr.start;
-        const double iphi = (double)(k + 1);
-        double phi;
-        if (sr.cap) phi = (iphi - 0.5) * kHalfPi / (double)sr.ipole;
-        else phi = (iphi - sr.pf) * kPi * 0.75 * e.fact1;
         double sp, cp;
-        sincos(phi, &sp, &cp);
+        if (sr.trig) {
+            const double2 t = __ldg(sr.trig + k);
+            sp = t.x;
+            cp = t.y;
+        } else {
+            sincos(sr.cap ? cap_phi(k, sr.ipole) : belt_phi(k, sr.pf, e.fact1), &sp, &cp);
+        }
         px = sr.st * cp;
         py = sr.st * sp;
         pz = sr.z;
     }
 
-    // src/genmap.cpp:135-143
+    // src/genmap.cpp:135-143: the weight of angular distance alpha
+    __device__ static double weight_at(const Ext &e, double alpha) {
+        constexpr double kR = 1.0 / 0.333;
+        double d2 = div_by(alpha, e.ar, e.inv_ar);
+        d2 = d2 * d2;
+        return exp(div_by(-0.5 * d2, 0.333, kR));
+    }
     __device__ static double weight(const Ext &e, const SegReg &sr, int pix) {
         double px, py, pz;
         pixel_vec(e, sr, pix, px, py, pz);
         const double dot = px * e.vx + py * e.vy + pz * e.vz;
-        const double dc = fmin(1.0, fmax(-1.0, dot));
-        double d2 = acos(dc) / e.ar;
-        d2 = d2 * d2;
-        return exp(-0.5 * d2 / 0.333);
+        return weight_at(e, acos(fmin(1.0, fmax(-1.0, dot))));
     }
 
-    __device__ static void norm_add(const Ext &e, const SegReg &sr, int j, int pix, NormAcc &acc) {
-        (void)j;
-        acc.s += weight(e, sr, pix);
-    }
-    __device__ static double norm_value(const NormAcc &acc) { return acc.s; }
-
-    __device__ static void deposit_setup(const DiscArgs &a, const DiscHdr &d, const Ext &e, double S,
-                                         Dep &dep) {
-        (void)a;
-        (void)e;
+    __device__ static void deposit_setup(const DiscHdr &d, double S, Dep &dep) {
         dep.S = S;
+        dep.inv_S = __ddiv_rn(1.0, S);
         dep.flux = d.flux;
     }
-    __device__ static void deposit(const DiscArgs &a, const Ext &e, const Dep &dep, const SegReg &sr,
-                                   int j, int pix) {
-        (void)j;
-        const double w = weight(e, sr, pix);
-        red_add_f64(a.acc.acc64 + pix, (w / dep.S) * dep.flux);
+    __device__ static void deposit(const DiscArgs &a, const Dep &dep, double w, int pix) {
+        red_add_f64(a.acc.acc64 + pix, div_by(w, dep.S, dep.inv_S) * dep.flux);
     }
     __device__ static void single(const DiscArgs &a, const DiscHdr &d) {
         red_add_f64(a.acc.acc64 + d.cpix, d.flux);
