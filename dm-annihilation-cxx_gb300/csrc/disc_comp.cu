@@ -344,13 +344,19 @@ __global__ void __launch_bounds__(kWPBA * 32) k_adjc_warp(adj::AdjArgs a) {
 
 // The headers of every disc in the queue, one thread per particle (the
 // FP64 set-up at full warp width instead of on one lane of a waiting block).
-__global__ void __launch_bounds__(256) k_comp_hdr(DiscArgs a) {
+// One warp per block: the FP64 set-up is bound by the FP64 pipe (a warp's
+// instruction takes 16 cycles of its SM's), so a few thousand discs are
+// spread over as many SMs as they fill warps (1000 discs: 23 us in blocks of
+// 256 threads, on 4 SMs).
+constexpr int kHdrWarps = 1;
+
+__global__ void __launch_bounds__(kHdrWarps * 32) k_comp_hdr(DiscArgs a) {
     // each warp builds its 32 consecutive headers in shared memory and
     // stores them as one contiguous run of 16-byte words (a thread's own
     // 160-byte store would leave partial sectors for the L2 to merge)
     constexpr int kW16 = sizeof(CompHdr) / 16;
     static_assert(sizeof(CompHdr) % 16 == 0, "headers are stored in 16-byte words");
-    __shared__ __align__(16) CompHdr stage[8][32];
+    __shared__ __align__(16) CompHdr stage[kHdrWarps][32];
     const long long ndisc = a.ctr[C_ADD_DISC];
     const long long stride = (long long)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -370,7 +376,7 @@ __global__ void __launch_bounds__(256) k_comp_hdr(DiscArgs a) {
 
 cudaError_t launch_hdr(const DiscArgs &a, int num_sms, cudaStream_t s) {
     if (!a.chdr) return cudaSuccess;
-    k_comp_hdr<<<num_sms * 8, 256, 0, s>>>(a);
+    k_comp_hdr<<<num_sms * 32, kHdrWarps * 32, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -6,6 +6,8 @@
 // flux, theta, phi, the angular radius and the centre pixel are those of
 // src/genmap.cpp:82-106 (with src/anglefuncs.cpp:15-52 and
 // src/flux/flux_ann_nosom.cpp:12-23).
+#include <cooperative_groups.h>
+
 #include "kernels.cuh"
 
 namespace dmann {
@@ -193,48 +195,68 @@ __global__ void __launch_bounds__(256) k_prep(PrepArgs a) {
     count_warp(a.ctr + C_DEPOSITS, single);
 }
 
-// Exclusive scan of the key histogram (one block); also publishes the
-// number of disc particles in the block-per-particle class.
-__global__ void __launch_bounds__(1024) k_scan(int *hist, long long *ctr, int block_bucket_min) {
-    constexpr int T = 1024, PER = kKeys / T;
+// Exclusive scan of the key histogram; also publishes the number of disc
+// particles in the block-per-particle class.  One cluster of kScanBlocks
+// blocks, 16 consecutive keys per thread in 16-byte words; the blocks' totals
+// meet in distributed shared memory.  (One block with 128 keys per thread
+// took 141 us, most of a small render.)
+constexpr int kScanBlocks = 8, kScanThreads = 1024, kScanPer = kKeys / (kScanBlocks * kScanThreads);
+static_assert(kScanPer == 16, "four 16-byte words per thread");
+
+__global__ void __cluster_dims__(kScanBlocks, 1, 1) __launch_bounds__(kScanThreads)
+    k_scan(int *hist, long long *ctr, int block_bucket_min) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
     __shared__ int wsum[32];
-    const int tid = threadIdx.x;
-    int local[PER];
-    int s = 0;
-#pragma unroll 8
-    for (int k = 0; k < PER; k++) {
-        local[k] = hist[tid * PER + k];
-        s += local[k];
+    __shared__ int total;
+    const int tid = threadIdx.x, rank = (int)cluster.block_rank();
+    const int key0 = (rank * kScanThreads + tid) * kScanPer;
+    int4 v[4];
+    int sum = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        v[k] = reinterpret_cast<const int4 *>(hist + key0)[k];
+        sum += v[k].x + v[k].y + v[k].z + v[k].w;
     }
     int tot;
-    int ex = warp_excl_scan(s, tot);
+    const int ex = warp_excl_scan(sum, tot);
     if ((tid & 31) == 0) wsum[tid >> 5] = tot;
     __syncthreads();
     if (tid < 32) {
         int t2;
-        int e2 = warp_excl_scan(wsum[tid], t2);
+        const int e2 = warp_excl_scan(wsum[tid], t2);
         wsum[tid] = e2;
+        if (tid == 0) total = t2;
     }
-    __syncthreads();
+    cluster.sync();
     int base = wsum[tid >> 5] + ex;
+    for (int r = 0; r < rank; r++) base += *cluster.map_shared_rank(&total, r);
     const int boundary_key = (kBuckets - block_bucket_min) * kCells;
-#pragma unroll 8
-    for (int k = 0; k < PER; k++) {
-        int key = tid * PER + k;
+    auto next = [&](int key, int &c) {
         if (key == boundary_key) {
             ctr[C_ADD_BLOCK] = base;
             ctr[C_DISC_BLOCK] += base;
         }
-        hist[key] = base;
-        base += local[k];
+        const int n = c;
+        c = base;
+        base += n;
+    };
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        next(key0 + 4 * k, v[k].x);
+        next(key0 + 4 * k + 1, v[k].y);
+        next(key0 + 4 * k + 2, v[k].z);
+        next(key0 + 4 * k + 3, v[k].w);
+        reinterpret_cast<int4 *>(hist + key0)[k] = v[k];
     }
-    if (tid == T - 1) {
+    if (rank == kScanBlocks - 1 && tid == kScanThreads - 1) {
         ctr[C_ADD_DISC] = base;
         if (boundary_key >= kKeys) {
             ctr[C_ADD_BLOCK] = base;
             ctr[C_DISC_BLOCK] += base;
         }
     }
+    cluster.sync();   // no block leaves while another reads its total
 }
 
 __global__ void __launch_bounds__(256) k_scatter(const int *key, int n, int *offsets, int *queue) {
@@ -270,12 +292,15 @@ __global__ void k_finalize(Accum acc, int precision, int npix, double dOmega, do
 
 cudaError_t launch_prep(const PrepArgs &a, cudaStream_t s) {
     if (a.p.n <= 0) return cudaSuccess;
-    k_prep<<<(a.p.n + 255) / 256, 256, 0, s>>>(a);
+    // small sets in blocks of one warp: the kernel is bound by the FP64 pipe,
+    // and 1000 particles in blocks of 256 keep 4 SMs busy (25 us)
+    const int bt = a.p.n <= 152 * 256 ? 32 : 256;
+    k_prep<<<(a.p.n + bt - 1) / bt, bt, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_scan(int *hist, long long *ctr, int block_bucket_min, cudaStream_t s) {
-    k_scan<<<1, 1024, 0, s>>>(hist, ctr, block_bucket_min);
+    k_scan<<<kScanBlocks, kScanThreads, 0, s>>>(hist, ctr, block_bucket_min);
     return cudaGetLastError();
 }
 
