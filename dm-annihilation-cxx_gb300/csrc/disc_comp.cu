@@ -27,22 +27,26 @@ __device__ void render_disc(const DiscArgs &a, CompSmem<RCH> &sm, const Ext &e) 
     // The offset is removed exactly after the pass.
     float2 ks = f2(1.0f), kc = f2(0.0f);
     long long total = 0;
+    int px = 0;   // of the staged chunk
     for (int c = 0; c < nchunk; c++) {
         const int r0 = r_first + c * RCH;
         const int n = min(RCH, r_last - r0 + 1);
-        total += build_runs<G, RCH>(a, sm, r0, n);
+        px = build_runs<G, RCH>(a, sm, r0, n);
+        total += px;
         if (G > 32) {
             if (rk == 0) sm.next_run = 0;
             Gp::sync();
         }
-        run_walk<G, RCH>(sm, n, [&](const Run &r, int, int j, bool second) {
+        auto add = [&](const Run &r, int, int j, int off, bool second) {
             const float jf = (float)j;
-            float2 w = weight2<TX, TH>(e, r, make_float2(jf, jf + 32.0f));
+            float2 w = weight2<TX, TH>(e, r, make_float2(jf, jf + (float)off));
             if (!second) w.y = 0.0f;
             const float2 t = add2(ks, w);
             kc = add2(kc, sub2(w, sub2(t, ks)));
             ks = t;
-        });
+        };
+        if constexpr (G == 32) warp_walk_any(sm, n, px, add);
+        else run_walk<G, RCH>(sm, n, add);
         Gp::sync();
     }
     if (total < 2) {  // genmap.cpp:125-128: the whole flux into the centre pixel
@@ -99,19 +103,21 @@ __device__ void render_disc(const DiscArgs &a, CompSmem<RCH> &sm, const Ext &e) 
     for (int c = 0; c < nchunk; c++) {
         const int r0 = r_first + c * RCH;
         const int n = min(RCH, r_last - r0 + 1);
-        if (nchunk > 1) build_runs<G, RCH>(a, sm, r0, n);
+        if (nchunk > 1) px = build_runs<G, RCH>(a, sm, r0, n);
         if (G > 32) {
             if (rk == 0) sm.next_run = 0;
             Gp::sync();
         }
-        run_walk<G, RCH>(sm, n, [&](const Run &r, int, int j, bool second) {
+        auto deposit = [&](const Run &r, int, int j, int off, bool second) {
             const float jf = (float)j;
-            const float2 w = weight2<TX, TH>(e, r, make_float2(jf, jf + 32.0f));
+            const float2 w = weight2<TX, TH>(e, r, make_float2(jf, jf + (float)off));
             const float2 p = fma2(w, f2(Fa), mul2(w, f2(Floa)));   // w |F|, rounded once
             double *const m = acc + (r.pix0 + j);
             red_add_f64(m, f32_to_f64(p.x, bias));
-            if (second) red_add_f64(m + 32, f32_to_f64(p.y, bias));
-        });
+            if (second) red_add_f64(m + off, f32_to_f64(p.y, bias));
+        };
+        if constexpr (G == 32) warp_walk_any(sm, n, px, deposit);
+        else run_walk<G, RCH>(sm, n, deposit);
         Gp::sync();
     }
 }
@@ -228,7 +234,7 @@ __device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long lon
             if (rk == 0) sm.c.next_run = 0;
             Gp::sync();
         }
-        run_walk<G, RCH>(sm.c, n, [&](const Run &r, int, int j, bool second) {
+        run_walk<G, RCH>(sm.c, n, [&](const Run &r, int, int j, int, bool second) {
             const float jf = (float)j;
             float2 w = weight2(e, r, make_float2(jf, jf + 32.0f));
             if (!second) w.y = 0.0f;
@@ -268,7 +274,7 @@ __device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long lon
             if (rk == 0) sm.c.next_run = 0;
             Gp::sync();
         }
-        run_walk<G, RCH>(sm.c, n, [&](const Run &r, int ring, int j, bool second) {
+        run_walk<G, RCH>(sm.c, n, [&](const Run &r, int ring, int j, int, bool second) {
             const float jf = (float)j;
             float2 sn, h, g;
             const float2 w = weight2x(e, r, make_float2(jf, jf + 32.0f), sn, h, g);

@@ -2,11 +2,10 @@
 dispatch, against the plain FP64 form on the same particles: the same set of
 non-zero pixels, the same deposit count, every pixel and the total flux.
 
-Tolerances.  A weight's exponent of 2 lies in [-8.7, 0] and comes from about
-six FP32 roundings of at most half an ulp (2.4e-7) each, so a deposit is off by
-less than 1.5e-6; a pixel adds FP32 sums of at most 512 deposits, whose
-rounding errors (at most 2^-24 of the sum each, of either sign) stay below
-1e-5.  The total flux is that of the per-particle normalisation, 1e-9 (the
+Tolerances.  A weight's exponent of 2, in [-8.7, 0], carries some 24 relative
+roundings of at most 2^-24 (test_gpu_disc_paths.py), 9e-6 of the weight; a
+pixel adds FP32 sums of at most 512 deposits, whose roundings have either sign:
+1e-5 per pixel.  The total flux is that of the per-particle normalisation, 1e-9 (the
 bound of the other tests); a single disc's normalisation comes from ring sums
 rounded to FP32 (6e-8 each, of either sign, over ten rings and more): 6e-8.
 """
