@@ -210,7 +210,7 @@ constexpr int kWPB = 8, kRCHW = 64;
 }  // namespace
 
 cudaError_t launch_adjoint(const DiscArgs &d, const Particles &p, const signed char *cls,
-                           const double *gmap, float *gmap32, double *grad, double *oacc,
+                           const double *gmap, float *gmap32, void *sum_buf, double *grad, double *oacc,
                            int precision, int num_sms, cudaStream_t s, const double *core_corr,
                            const double *core_gln) {
     AdjArgs a;
@@ -233,7 +233,7 @@ cudaError_t launch_adjoint(const DiscArgs &d, const Particles &p, const signed c
         if (blocks > num_sms * 16) blocks = num_sms * 16;
         k_to_f32<<<blocks, 256, 0, s>>>(gmap, gmap32, d.g.npix);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        return launch_adjoint_comp_discs(a, num_sms, s);
+        return launch_adjoint_comp_discs(a, sum_buf, num_sms, s);
     }
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adj_block<kBT, kRCH>, kBT, 0);

@@ -156,7 +156,8 @@ __device__ inline void flush_acc(double *oacc, const double acc[12]) {
 
 }  // namespace adj
 
-// disc_comp.cu: the compensated-FP32 adjoint's disc kernels
-cudaError_t launch_adjoint_comp_discs(const adj::AdjArgs &a, int num_sms, cudaStream_t s);
+// disc_comp.cu: the compensated-FP32 adjoint's disc kernels; sum_buf holds
+// kAdjSumBytes per particle
+cudaError_t launch_adjoint_comp_discs(const adj::AdjArgs &a, void *sum_buf, int num_sms, cudaStream_t s);
 
 }  // namespace dmann

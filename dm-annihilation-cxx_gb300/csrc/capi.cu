@@ -78,6 +78,7 @@ struct dmann_ctx {
     // per-map work (w: work[0], or a batch lane's)
     DevBuf in[7], map;
     DevBuf cls, oacc, grad;   // the adjoint's class array, observer sums, staged gradient
+    DevBuf adj_sums;          // the compensated adjoint's sums per disc
     DevBuf core_gln;          // the adjoint's d ln(halo-core factor) / d pos, [3][n]
     Work work[2];
     Work *w = &work[0];
@@ -414,7 +415,7 @@ void dmann_destroy(dmann_ctx *ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     DevBuf *bufs[] = {&ctx->in[0], &ctx->in[1], &ctx->in[2], &ctx->in[3], &ctx->in[4], &ctx->in[5],
-                      &ctx->in[6], &ctx->map, &ctx->cls, &ctx->oacc, &ctx->grad, &ctx->halo_f,
+                      &ctx->in[6], &ctx->map, &ctx->cls, &ctx->oacc, &ctx->grad, &ctx->adj_sums, &ctx->halo_f,
                       &ctx->halo_cells, &ctx->corr, &ctx->core_gln, &ctx->bstats};
     for (Work &wk : ctx->work) {
         DevBuf *wb[] = {&wk.theta, &wk.phi, &wk.ar, &wk.flux, &wk.cpix, &wk.key, &wk.queue, &wk.hist,
@@ -1438,7 +1439,7 @@ dmann_status dmann_adjoint_v(dmann_ctx *ctx, const float *x, const float *y, con
     if (core && ((st = ensure(ctx, ctx->corr, 8 * n1)) || (st = ensure(ctx, ctx->core_gln, 24 * n1))))
         return st;
     if (precision == DMANN_COMP_F32) {
-        if ((st = ensure(ctx, ctx->w->acc, 4 * P)) != DMANN_OK) return st;
+        if ((st = ensure(ctx, ctx->w->acc, 4 * P)) || (st = ensure(ctx, ctx->adj_sums, kAdjSumBytes * n1))) return st;
         reserve_headers(ctx, n1);
     } else {
         reserve_plain(ctx, nside);
@@ -1512,7 +1513,7 @@ dmann_status dmann_adjoint_v(dmann_ctx *ctx, const float *x, const float *y, con
     if (precision == DMANN_COMP_F32) da.chdr = headers_for(ctx, n1);
     else plain_args(ctx, nside, da);
     CK(cudaEventRecord(ctx->evd0, s));
-    CK(launch_adjoint(da, pa.p, pa.out.cls, dgmap, (float *)ctx->w->acc.p, dgrad, (double *)ctx->oacc.p,
+    CK(launch_adjoint(da, pa.p, pa.out.cls, dgmap, (float *)ctx->w->acc.p, ctx->adj_sums.p, dgrad, (double *)ctx->oacc.p,
                       precision, ctx->num_sms, s, core ? (const double *)ctx->corr.p : nullptr,
                       core ? (const double *)ctx->core_gln.p : nullptr));
     CK(cudaEventRecord(ctx->evd1, s));

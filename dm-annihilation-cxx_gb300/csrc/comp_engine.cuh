@@ -559,19 +559,21 @@ __device__ inline int build_runs(const DiscArgs &a, CompSmem<RCH> &sm, int r0, i
     return c;
 }
 
-// A warp on the staged rings with S lanes per ring, 32 / S rings at a time:
-// lane l of a ring's group handles pixels l and l + S of each 2 S of a run;
-// body as in run_walk with off = S.
+// One run with S lanes (sl: this one): pixels j and j + S of each 2 S.
+template <int S, class Body>
+__device__ __forceinline__ void lane_walk(const Run &r, int q, int sl, Body body) {
+    for (int j = sl; j < r.cnt; j += 2 * S) body(r, q, j, S, j + S < r.cnt);
+}
+
+// A warp on the staged rings with S lanes per ring, 32 / S rings at a time;
+// body as in sum_walk.
 template <int S, int RCH, class Body>
 __device__ inline void warp_walk(CompSmem<RCH> &sm, int n, Body body) {
     const int lane = threadIdx.x & 31, sl = lane % S;
     for (int q = lane / S; q < n; q += 32 / S) {
         const Run r = sm.run[2 * q];
-        for (int j = sl; j < r.cnt; j += 2 * S) body(r, q, j, S, j + S < r.cnt);
-        if (r.more) {
-            const Run r2 = sm.run[2 * q + 1];
-            for (int j = sl; j < r2.cnt; j += 2 * S) body(r2, q, j, S, j + S < r2.cnt);
-        }
+        lane_walk<S>(r, q, sl, body);
+        if (r.more) lane_walk<S>(sm.run[2 * q + 1], q, sl, body);
     }
     __syncwarp();
 }
@@ -588,37 +590,62 @@ __device__ inline void warp_walk_any(CompSmem<RCH> &sm, int n, int px, Body body
     else warp_walk<32>(sm, n, body);
 }
 
-// Walks the staged rings; lane l handles pixels l and l + off (32) of each
-// 64-pixel stretch of a run.  body(run, ring, j, off, second) gets the ring's
-// index in the chunk, the first pixel index j and whether j + off is inside
-// the run.  In a block, warps claim whole
-// rings (both run slots: the second only when the ring wrapped) from a shared
-// counter reset by the caller; the next claim is issued before the current
-// ring is walked, so its latency is hidden, and no warp waits at the next
-// barrier for more than about one ring.
-template <int G, int RCH, class Body>
-__device__ inline void run_walk(CompSmem<RCH> &sm, int n, Body body) {
-    const int lane = threadIdx.x & 31;
-    auto ring = [&](int i) {
-        const Run r = sm.run[2 * i];
-        for (int j = lane; j < r.cnt; j += 64) body(r, i, j, 32, j + 32 < r.cnt);
-        if (r.more) {
-            const Run r2 = sm.run[2 * i + 1];
-            for (int j = lane; j < r2.cnt; j += 64) body(r2, i, j, 32, j + 32 < r2.cnt);
-        }
-    };
-    if (G == 32) {
-        for (int i = 0; i < n; i++) ring(i);
-        return;
-    }
-    int q = 0;
-    if (lane == 0) q = atomicAdd(&sm.next_run, 1);
-    q = __shfl_sync(0xffffffffu, q, 0);
-    while (q < n) {
+// The warps of a block on the staged rings, S lanes per ring: a warp claims
+// 32 / S rings at a time from a shared-memory counter reset by the caller; the
+// next claim is issued before the current rings are walked, so its latency is
+// hidden, and no warp waits at the next barrier for more than about one claim.
+template <int S, int RCH, class Body>
+__device__ inline void block_walk(CompSmem<RCH> &sm, int n, Body body) {
+    const int lane = threadIdx.x & 31, sl = lane % S;
+    int q0 = 0;
+    if (lane == 0) q0 = atomicAdd(&sm.next_run, 32 / S);
+    q0 = __shfl_sync(0xffffffffu, q0, 0);
+    while (q0 < n) {
         int qn = 0;
-        if (lane == 0) qn = atomicAdd(&sm.next_run, 1);
-        ring(q);
-        q = __shfl_sync(0xffffffffu, qn, 0);
+        if (lane == 0) qn = atomicAdd(&sm.next_run, 32 / S);
+        const int q = q0 + lane / S;
+        if (q < n) {
+            const Run r = sm.run[2 * q];
+            lane_walk<S>(r, q, sl, body);
+            if (r.more) lane_walk<S>(sm.run[2 * q + 1], q, sl, body);
+        }
+        q0 = __shfl_sync(0xffffffffu, qn, 0);
+    }
+}
+
+// Walks the n staged rings (px pixels): body(run, ring, j, off, second) gets
+// the ring's index in the chunk, a pixel index j, and whether j + off is inside
+// the run too.  sum_walk: the body reads or sums, so few lanes share a ring
+// (short steps waste few lanes at a run's end, and a ring's set-up is shared by
+// the rings a warp walks together), as long as every warp has rings.
+// deposit_walk: the body deposits, so the lanes are fitted to the rings' mean
+// length and stay on consecutive pixels.
+template <int G, int RCH, class Body>
+__device__ inline void sum_walk(CompSmem<RCH> &sm, int n, int px, Body body) {
+    if constexpr (G == 32) {
+        warp_walk_any(sm, n, px, body);
+    } else {
+        if (n >= G / 8) block_walk<8>(sm, n, body);
+        else if (n >= G / 16) block_walk<16>(sm, n, body);
+        else block_walk<32>(sm, n, body);
+    }
+}
+
+// A ring per warp at a time (the adjoint, whose signed sums' roundings depend
+// on how the pixels are dealt to the lanes).
+template <int G, int RCH, class Body>
+__device__ inline void ring_walk(CompSmem<RCH> &sm, int n, Body body) {
+    if constexpr (G == 32) warp_walk<32>(sm, n, body);
+    else block_walk<32>(sm, n, body);
+}
+
+template <int G, int RCH, class Body>
+__device__ inline void deposit_walk(CompSmem<RCH> &sm, int n, int px, Body body) {
+    if constexpr (G == 32) {
+        warp_walk_any(sm, n, px, body);
+    } else {
+        if (n >= G / 16 && px <= 96 * n) block_walk<16>(sm, n, body);
+        else block_walk<32>(sm, n, body);
     }
 }
 

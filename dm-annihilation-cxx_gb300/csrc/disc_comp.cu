@@ -45,8 +45,7 @@ __device__ void render_disc(const DiscArgs &a, CompSmem<RCH> &sm, const Ext &e) 
             kc = add2(kc, sub2(w, sub2(t, ks)));
             ks = t;
         };
-        if constexpr (G == 32) warp_walk_any(sm, n, px, add);
-        else run_walk<G, RCH>(sm, n, add);
+        sum_walk<G, RCH>(sm, n, px, add);
         Gp::sync();
     }
     if (total < 2) {  // genmap.cpp:125-128: the whole flux into the centre pixel
@@ -116,8 +115,7 @@ __device__ void render_disc(const DiscArgs &a, CompSmem<RCH> &sm, const Ext &e) 
             red_add_f64(m, f32_to_f64(p.x, bias));
             if (second) red_add_f64(m + off, f32_to_f64(p.y, bias));
         };
-        if constexpr (G == 32) warp_walk_any(sm, n, px, deposit);
-        else run_walk<G, RCH>(sm, n, deposit);
+        deposit_walk<G, RCH>(sm, n, px, deposit);
         Gp::sync();
     }
 }
@@ -192,14 +190,39 @@ cudaError_t launch_block(const DiscArgs &a, int num_sms, int blocks_per_sm, cuda
 // difference v - cos(alpha) n is not); alpha / sin(alpha) =
 // sqrt(g / (h (1 - h))) with h = hav(alpha) and g = alpha^2 / 4 from the
 // weight.  Sums: S with the offset Fast2Sum, the signed ones (sum G w, V_theta,
-// V_phi, T) with Kahan's compensation per lane, all reduced in FP64; the
-// epilogue turns V into the map frame and writes the gradient in FP64.
+// V_phi, T) with Kahan's compensation per lane, all reduced as two-floats; a
+// kernel with one thread per disc turns V into the map frame and writes the
+// gradient in FP64.
 template <int RCH>
 struct AdjcSmem {
     CompSmem<RCH> c;
     AdjRing aring[RCH];
-    double red[3][32];
+    float2 red[5][32];
 };
+
+// A disc's sums over its pixels: S, sum G w, V_theta, V_phi, T (S = 0: fewer
+// than two pixels).
+struct AdjSums {
+    double S, A, vt, vp, t;
+};
+static_assert(sizeof(AdjSums) == kAdjSumBytes, "the caller's buffer");
+
+// Two-float sum over the group; every thread ends with the total.  red: one
+// slot per warp, used for nothing else within a disc.
+template <int G>
+__device__ __forceinline__ void group_sum_ff(float2 &v, float2 *red) {
+    warp_sum_ff(v.x, v.y);
+    if (G > 32) {
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        v = red[0];
+        for (int w = 1; w < G / 32; w++) {
+            float err;
+            v.x = two_sum(v.x, red[w].x, err);
+            v.y = (v.y + red[w].y) + err;
+        }
+    }
+}
 
 __device__ __forceinline__ void kahan(float &s, float &c, float v) {
     const float y = v - c;
@@ -209,13 +232,12 @@ __device__ __forceinline__ void kahan(float &s, float &c, float v) {
 }
 
 template <int G, int RCH>
-__device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long long q, double acc[12]) {
+__device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long long q, AdjSums *sums) {
     using Gp = Grp<G>;
     const DiscArgs &da = a.d;
     const int rk = Gp::rank();
     stage_hdr<G>(da, q, sm.c.h);
     Gp::sync();
-    const int pidx = sm.c.h.hdr.pidx;
     const Ext e = sm.c.h.ext;
     const int r_first = sm.c.h.hdr.r_first, r_last = sm.c.h.hdr.r_last;
     const int nring = r_last - r_first + 1;
@@ -234,12 +256,12 @@ __device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long lon
             if (rk == 0) sm.c.next_run = 0;
             Gp::sync();
         }
-        run_walk<G, RCH>(sm.c, n, [&](const Run &r, int, int j, int, bool second) {
+        ring_walk<G, RCH>(sm.c, n, [&](const Run &r, int, int j, int off, bool second) {
             const float jf = (float)j;
-            float2 w = weight2(e, r, make_float2(jf, jf + 32.0f));
+            float2 w = weight2(e, r, make_float2(jf, jf + (float)off));
             if (!second) w.y = 0.0f;
             const int pix = r.pix0 + j;
-            const float gw = g32[pix] * w.x + (second ? g32[pix + 32] * w.y : 0.0f);
+            const float gw = g32[pix] * w.x + (second ? g32[pix + off] * w.y : 0.0f);
             kahan(as, ac, gw);
             const float2 t = add2(ks, w);
             kc = add2(kc, sub2(w, sub2(t, ks)));
@@ -247,22 +269,28 @@ __device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long lon
         });
         Gp::sync();
     }
-    double s1[3] = {(((double)ks.x - 1.0) + (double)kc.x) + (((double)ks.y - 1.0) + (double)kc.y),
-                    (double)as - (double)ac, 0.0};
-    adj::group_sum<G, 2>(s1, sm.red);
+    // (ks - 1 is exact, and so are the error terms of the two-float trees: no
+    // FP64, whose pipe -- 1/64 of the FP32 rate -- was 73 % busy with these
+    // sums in every warp and the epilogue on one lane per disc)
+    float err;
+    float2 S2, A2;
+    S2.x = two_sum(ks.x - 1.0f, ks.y - 1.0f, err);
+    S2.y = (kc.x + kc.y) + err;
+    A2 = make_float2(as, -ac);
+    group_sum_ff<G>(S2, sm.red[0]);
+    group_sum_ff<G>(A2, sm.red[1]);
+    AdjSums &out = sums[q];
     if (total < 2) {  // genmap.cpp:125-128: the whole flux in the centre pixel
         if (rk == 0) {
-            const double KV[3] = {0.0, 0.0, 0.0};
-            adj::write_grad(a, pidx, a.gmap[sm.c.h.hdr.cpix] * a.inv_dOmega, 0.0, KV, false, acc);
+            out.S = 0.0;
             atomicAdd((unsigned long long *)(da.ctr + C_DEPOSITS), 1ull);
         }
         Gp::sync();
         return;
     }
     if (rk == 0) atomicAdd((unsigned long long *)(da.ctr + C_DEPOSITS), (unsigned long long)total);
-    const double S = s1[0];
-    const double Gm = s1[1] / S;
-    const float gm = (float)Gm;
+    const float2 gq = div_ff(A2.x, A2.y, S2.x, S2.y);
+    const float gm = gq.x;   // sum G w / S rounded
 
     // pass 2: V_theta, V_phi, T with q = (G - Gm) w
     float vts = 0.0f, vtc = 0.0f, vps = 0.0f, vpc = 0.0f, ts = 0.0f, tc = 0.0f;
@@ -274,10 +302,10 @@ __device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long lon
             if (rk == 0) sm.c.next_run = 0;
             Gp::sync();
         }
-        run_walk<G, RCH>(sm.c, n, [&](const Run &r, int ring, int j, int, bool second) {
+        ring_walk<G, RCH>(sm.c, n, [&](const Run &r, int ring, int j, int off, bool second) {
             const float jf = (float)j;
             float2 sn, h, g;
-            const float2 w = weight2x(e, r, make_float2(jf, jf + 32.0f), sn, h, g);
+            const float2 w = weight2x(e, r, make_float2(jf, jf + (float)off), sn, h, g);
             const AdjRing ar = sm.aring[ring];
             const int pix = r.pix0 + j;
             float vt = 0.0f, vp = 0.0f, tt = 0.0f;
@@ -286,7 +314,7 @@ __device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long lon
                 if (k == 1 && !second) break;
                 const float wk = k ? w.y : w.x, snk = k ? sn.y : sn.x, hk = k ? h.y : h.x,
                             gk = k ? g.y : g.x;
-                const float q = (g32[pix + 32 * k] - gm) * wk;
+                const float q = (g32[k ? pix + off : pix] - gm) * wk;
                 // alpha / sin(alpha); 0 at the antipode, where the tangent is undefined
                 const float om = 1.0f - hk;
                 const float af = hk > 1e-30f ? (om > 1e-7f ? sqrtf(gk / (hk * om)) : 0.0f) : 1.0f;
@@ -304,24 +332,62 @@ __device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long lon
         });
         Gp::sync();
     }
-    double s2[3] = {(double)vts - (double)vtc, (double)vps - (double)vpc, (double)ts - (double)tc};
-    adj::group_sum<G, 3>(s2, sm.red);
+    float2 vt = make_float2(vts, -vtc), vp = make_float2(vps, -vpc), tt = make_float2(ts, -tc);
+    group_sum_ff<G>(vt, sm.red[2]);
+    group_sum_ff<G>(vp, sm.red[3]);
+    group_sum_ff<G>(tt, sm.red[4]);
     if (rk == 0) {
-        const DiscHdr &d = sm.c.h.hdr;
-        const double ct = cos(d.theta0), st = sin(d.theta0), cp = cos(d.phi0), sp = sin(d.phi0);
-        const double V[3] = {s2[0] * ct * cp - s2[1] * sp, s2[0] * ct * sp + s2[1] * cp, -s2[0] * st};
-        const double K = adj::kInvC2 * d.flux / (S * d.ar * d.ar) * a.inv_dOmega;
-        const double KV[3] = {K * V[0], K * V[1], K * V[2]};
-        adj::write_grad(a, pidx, Gm * a.inv_dOmega, K * s2[2], KV, true, acc);
+        out.S = (double)S2.x + (double)S2.y;
+        out.A = (double)A2.x + (double)A2.y;
+        out.vt = (double)vt.x + (double)vt.y;
+        out.vp = (double)vp.x + (double)vp.y;
+        out.t = (double)tt.x + (double)tt.y;
     }
     Gp::sync();
 }
 
+// The gradients of the disc particles from their sums (FP64), one thread per
+// disc, and the observer terms.
+__global__ void __launch_bounds__(128) k_adjc_grad(adj::AdjArgs a, const AdjSums *sums) {
+    __shared__ double red[12][32];
+    double acc[12] = {0.0};
+    const long long ndisc = a.d.ctr[C_ADD_DISC];
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < ndisc; q += (long long)gridDim.x * blockDim.x) {
+        const AdjSums s = sums[q];
+        const int i = a.d.queue[q];
+        if (s.S == 0.0) {
+            const double KV[3] = {0.0, 0.0, 0.0};
+            adj::write_grad(a, i, a.gmap[a.d.cpix[i]] * a.inv_dOmega, 0.0, KV, false, acc);
+            continue;
+        }
+        double theta0, phi0, ar;
+        if (a.d.chdr) {
+            const DiscHdr &d = a.d.chdr[q].hdr;
+            theta0 = d.theta0;
+            phi0 = d.phi0;
+            ar = d.ar;
+        } else {
+            DiscHdr d;
+            disc_setup(a.d.g, a.d.theta[i], a.d.phi[i], a.d.ar[i], a.d.flux[i], a.d.cpix[i], i, d);
+            theta0 = d.theta0;
+            phi0 = d.phi0;
+            ar = d.ar;
+        }
+        const double Gm = s.A / s.S;
+        const double ct = cos(theta0), st = sin(theta0), cp = cos(phi0), sp = sin(phi0);
+        const double V[3] = {s.vt * ct * cp - s.vp * sp, s.vt * ct * sp + s.vp * cp, -s.vt * st};
+        const double K = adj::kInvC2 * a.d.flux[i] / (s.S * ar * ar) * a.inv_dOmega;
+        const double KV[3] = {K * V[0], K * V[1], K * V[2]};
+        adj::write_grad(a, i, Gm * a.inv_dOmega, K * s.t, KV, true, acc);
+    }
+    adj::group_sum<128, 12>(acc, red);
+    if (threadIdx.x == 0) adj::flush_acc(a.oacc, acc);
+}
+
 template <int BT, int RCH, int MINB>
-__global__ void __launch_bounds__(BT, MINB) k_adjc_block(adj::AdjArgs a) {
+__global__ void __launch_bounds__(BT, MINB) k_adjc_block(adj::AdjArgs a, AdjSums *sums) {
     __shared__ AdjcSmem<RCH> sm;
     __shared__ int s_q;
-    double acc[12] = {0.0};
     const long long nblk = a.d.ctr[C_ADD_BLOCK];
     for (;;) {
         if (threadIdx.x == 0) s_q = (int)atomicAdd((unsigned long long *)(a.d.ctr + C_QNEXT_BLOCK), 1ull);
@@ -329,23 +395,20 @@ __global__ void __launch_bounds__(BT, MINB) k_adjc_block(adj::AdjArgs a) {
         const int q = s_q;
         __syncthreads();
         if (q >= nblk) break;
-        adjc_particle<BT, RCH>(a, sm, q, acc);
+        adjc_particle<BT, RCH>(a, sm, q, sums);
     }
-    if (threadIdx.x == 0) adj::flush_acc(a.oacc, acc);
 }
 
 constexpr int kWPBA = 4;   // warps per block of the adjoint's warp kernel (shared memory)
 
-__global__ void __launch_bounds__(kWPBA * 32) k_adjc_warp(adj::AdjArgs a) {
+__global__ void __launch_bounds__(kWPBA * 32) k_adjc_warp(adj::AdjArgs a, AdjSums *sums) {
     __shared__ AdjcSmem<kRCHW> sm[kWPBA];
-    double acc[12] = {0.0};
     const long long nblk = a.d.ctr[C_ADD_BLOCK];
     const long long ndisc = a.d.ctr[C_ADD_DISC];
     const int w = threadIdx.x >> 5;
     const long long gw = (long long)blockIdx.x * kWPBA + w;
     const long long nw = (long long)gridDim.x * kWPBA;
-    for (long long q = nblk + gw; q < ndisc; q += nw) adjc_particle<32, kRCHW>(a, sm[w], q, acc);
-    if ((threadIdx.x & 31) == 0) adj::flush_acc(a.oacc, acc);
+    for (long long q = nblk + gw; q < ndisc; q += nw) adjc_particle<32, kRCHW>(a, sm[w], q, sums);
 }
 
 // The headers of every disc in the queue, one thread per particle (the
@@ -422,20 +485,23 @@ cudaError_t launch_disc_comp(const DiscArgs &a, int num_sms, int blocks_per_sm, 
 }
 
 // The compensated adjoint's disc kernels (block class, then warp class).
-cudaError_t launch_adjoint_comp_discs(const adj::AdjArgs &a, int num_sms, cudaStream_t s) {
+cudaError_t launch_adjoint_comp_discs(const adj::AdjArgs &a, void *sum_buf, int num_sms, cudaStream_t s) {
+    AdjSums *const sums = (AdjSums *)sum_buf;
     cudaError_t e = launch_hdr(a.d, num_sms, s);
     if (e != cudaSuccess) return e;
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adjc_block<256, 256, 4>, 256, 0);
     if (e != cudaSuccess) return e;
     if (occ < 1) occ = 1;
-    k_adjc_block<256, 256, 4><<<num_sms * occ, 256, 0, s>>>(a);
+    k_adjc_block<256, 256, 4><<<num_sms * occ, 256, 0, s>>>(a, sums);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int occw = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occw, k_adjc_warp, kWPBA * 32, 0);
     if (e != cudaSuccess) return e;
     if (occw < 1) occw = 1;
-    k_adjc_warp<<<num_sms * occw, kWPBA * 32, 0, s>>>(a);
+    k_adjc_warp<<<num_sms * occw, kWPBA * 32, 0, s>>>(a, sums);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    k_adjc_grad<<<num_sms * 8, 128, 0, s>>>(a, sums);
     return cudaGetLastError();
 }
 

@@ -249,9 +249,11 @@ cudaError_t launch_disc_comp_block(const DiscArgs &a, int num_sms, int blocks_pe
 // sum_i dL/du_i and dL/drot (row-major).  Needs the prep outputs (with cls)
 // and the disc queue of the same particles and frame.
 // precision: DMANN_PLAIN_F64 (FP64 weights) or DMANN_COMP_F32 (the
-// compensated form's FP32 weights; gmap32 receives gmap rounded, npix floats).
+// compensated form's FP32 weights; gmap32 receives gmap rounded, npix floats;
+// sum_buf has kAdjSumBytes per particle).
+constexpr size_t kAdjSumBytes = 40;
 cudaError_t launch_adjoint(const DiscArgs &d, const Particles &p, const signed char *cls,
-                           const double *gmap, float *gmap32, double *grad, double *oacc,
+                           const double *gmap, float *gmap32, void *sum_buf, double *grad, double *oacc,
                            int precision, int num_sms, cudaStream_t s,
                            const double *core_corr = nullptr, const double *core_gln = nullptr);
 
