@@ -743,9 +743,9 @@ bool have_tile(dmann_ctx *ctx, size_t n, int nside, bool grow) {
     const size_t n1 = n > 0 ? n : 1, nt = (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
     return have_opt(w.seg_S, 8 * n1, grow) && have_opt(w.seg_px, 8 * n1, grow) &&
            have_opt(w.seg_cls, kSegBufBytes, grow) && have_opt(w.tile_gen, 4 * n1, grow) && have_opt(w.tile_hdr, sizeof(TileHdr) * n1, grow) &&
-           have_opt(w.tile_hist, 3 * nt * kTileClasses * sizeof(unsigned), grow) &&
-           have_opt(w.tile_base, 3 * nt * sizeof(long long), grow) &&
-           have_opt(w.tile_units, 3 * tile_unit_capacity(n, nside) * sizeof(TileUnit), grow) &&
+           have_opt(w.tile_hist, kTileLists * nt * kTileClasses * sizeof(unsigned), grow) &&
+           have_opt(w.tile_base, kTileLists * nt * sizeof(long long), grow) &&
+           have_opt(w.tile_units, kTileLists * tile_unit_capacity(n, nside) * sizeof(TileUnit), grow) &&
            have_opt(w.tile_list, 4 * tile_capacity(n, nside), grow);
 }
 
@@ -836,7 +836,7 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     tg.hdr = (TileHdr *)w.tile_hdr.p;
     CK(cudaMemsetAsync(buf, 0, kSegBufBytes, s));
     if (tile)
-        CK(cudaMemsetAsync(w.tile_hist.p, 0, 3 * (size_t)tg.nstrips * tg.ncol * kTileClasses * sizeof(unsigned), s));
+        CK(cudaMemsetAsync(w.tile_hist.p, 0, kTileLists * (size_t)tg.nstrips * tg.ncol * kTileClasses * sizeof(unsigned), s));
     CK(launch_hdr(da, ctx->num_sms, s));
     CK(launch_seg_count(da, sg, bt, ctx->num_sms, s));
     if (tile) CK(launch_tile_hdr(da, tg, seg, ctx->num_sms, s));
@@ -847,7 +847,7 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     if (timed) CK(cudaEventRecord(ctx->evp1, s));
     if (tile) {
         CK(launch_tile_deposits(da, tg, ctx->num_sms, s));
-        ctx->launches += 10 + (seg ? 1 : 0);
+        ctx->launches += 11 + (seg ? 1 : 0);
     }
     if (seg) {
         w.plane_clean = false;

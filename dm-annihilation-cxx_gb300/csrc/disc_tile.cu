@@ -4,6 +4,9 @@
 // A deposit per disc pixel is one reduction in L2, and at full overlap
 // density those reductions bound a scatter (disc_seg.cu: 1.07e12 deposits/s
 // on the 16M-particle workload, 0.75 of a bare sweep of FP32 reductions).
+// Times below are of 1M of the 16M set's particles at Nside 2048 (4.6e10
+// deposits): 36 ms in all.  The whole set takes 0.60 s, and 1.22 s by the
+// segmented render.
 // Here a warp owns a tile of the map -- 32 rings (one per lane) by kTileW
 // in-ring pixel indices -- in registers, and walks the list of the discs
 // that touch it: the sums never leave the SM until the tile is flushed, with
@@ -11,14 +14,14 @@
 //
 // Sequence (one stream, nothing waits for the host):
 //   k_tile_total    (disc, tile) pairs of the chunk, for its mode
-//   k_tile_norm     weight sums S of the polynomial discs; k_tile_norm_gen of
-//                   the others
+//   k_tile_norm     weight sums S of the discs; k_tile_norm_giant
+//                   of the largest
 //   k_tile_fin      F = flux / S per disc, discs of fewer than two pixels
 //   k_tile_pairs<1> pairs per (tile, octave of F)
 //   k_tile_plan     each tile's range of the pair list, its octaves in
 //                   ascending order, cut into work units
 //   k_tile_pairs<2> the pair list
-//   k_tile_dep<0>   units of polynomial discs; <1>, k_tile_dep_px of the others
+//   k_tile_dep<0>, <1> units of polynomial discs; <2>, k_tile_dep_px of the others
 //
 // Weight sums without visiting the pixels.  Along a ring the weight is a
 // smooth even function f(x) of the half azimuth offset x (a Gaussian, cut at
@@ -53,12 +56,21 @@ static_assert(kCls == kTileClasses, "histogram size");
 
 // How a disc's weights are evaluated.
 enum Kind {
-    K_POLY = 0,    // the ring's exponent polynomial
-    K_GEN = 1,     // run-time series per value
-    K_GIANT = 2    // the same; radius beyond kGiantR, which may reach the kink at the antipode
+    K_POLY3 = 0,   // the ring's exponent polynomial without its y^4 term
+    K_POLY = 1,    // the ring's exponent polynomial
+    K_GEN = 2,     // run-time series per value
+    K_GIANT = 3    // the same; radius beyond kGiantR, which may reach the kink at the antipode
 };
 constexpr int kKindMask = 3, kFlagH1 = 4, kFlagAll = 8, kFlagFast = 16, kFlagA2 = 32;
 constexpr double kGiantR = 2.2;
+
+// The y^4 term is at most 2.7e-8 in the exponent of 2 for half azimuth offsets
+// x below 0.1 rad (y = x^2) and the three-term asin^2 tier (h < 4e-3): a ninth
+// of the exponent's FP32 rounding.  sin R / sin theta0 = sin 2x at x = 0.1.
+// Without it the 16M workload takes 604 ms instead of 632; the maps' error
+// against the FP64 form is the same (Nside 512: 4.8e-8 with, 5.5e-8 without;
+// 2048: 8.1e-8 and 8.0e-8, 1.06e-7 and 1.06e-7).
+constexpr float kPoly3Sin = 0.1987f;
 
 // Rings from which a general disc's exponent is interpolated over 32 pixels
 // (half azimuth offsets of 16 pixels below 0.06 rad: see add_gen).
@@ -224,9 +236,15 @@ __device__ constexpr float kGwGLo[kNodesGen] = {1.0278e-09f, 6.3130e-09f, 1.3962
 constexpr int kDirect = 24, kDirectGen = 64;   // pixels up to which a ring is summed pixel by pixel
 constexpr int kFullPts = 32;                   // points of a full ring's trapezoid rule
 
+template <bool P3 = false>
 __device__ __forceinline__ float2 poly_exp2(const float c[5], float2 y) {
-    float2 t = fma2(y, f2(c[4]), f2(c[3]));
-    t = fma2(y, t, f2(c[2]));
+    float2 t;
+    if constexpr (P3) {
+        t = fma2(y, f2(c[3]), f2(c[2]));
+    } else {
+        t = fma2(y, f2(c[4]), f2(c[3]));
+        t = fma2(y, t, f2(c[2]));
+    }
     t = fma2(y, t, f2(c[1]));
     return fma2(y, t, f2(c[0]));
 }
@@ -420,8 +438,10 @@ __global__ void __launch_bounds__(256) k_tile_hdr(DiscArgs a, TileArgs tg) {
         t.irmax = c.hdr.irmax;
         t.q = (int)q;
         int kind;
-        if (c.ext.tier_x < 2 && c.ext.tier_h < 2) kind = K_POLY;
-        else kind = c.hdr.R < kGiantR ? K_GEN : K_GIANT;
+        if (c.ext.tier_x < 2 && c.ext.tier_h < 2)
+            kind = c.ext.tier_h == 0 && sinf((float)c.hdr.R) < kPoly3Sin * c.ch.sth0 ? K_POLY3 : K_POLY;
+        else
+            kind = c.hdr.R < kGiantR ? K_GEN : K_GIANT;
         t.flags = kind | (c.ext.tier_h >= 1 ? kFlagH1 : 0) | (c.hdr.allsky ? kFlagAll : 0) |
                   (c.ch.fast ? kFlagFast : 0) | (c.ext.tier_h == 2 ? kFlagA2 : 0);
         tg.hdr[q] = t;
@@ -454,7 +474,9 @@ constexpr int kNormWarps = 4;
 constexpr int kNormClaim = 4;   // discs per claim
 
 // S and the pixel count of every disc but the giants: a warp per disc, a ring
-// per lane.
+// per lane.  5.6 ms, bound by FP32 issue (the ring's chord test and 8 or 12
+// node values; the segmented render's first pass visits every pixel: 0.41 s
+// on the whole set).
 __global__ void __launch_bounds__(kNormWarps * 32, 7)
     k_tile_norm(const __grid_constant__ DiscArgs a, const __grid_constant__ TileArgs tg) {
     if (tg.ctl[0] != 2) return;
@@ -480,7 +502,7 @@ __global__ void __launch_bounds__(kNormWarps * 32, 7)
             float s = 0.0f, c = 0.0f;
             int total = 0;
             const int r_last = h.r_last;
-            if (kind == K_POLY) {
+            if (kind <= K_POLY) {
                 const int th = (h.flags & kFlagH1) ? 1 : 0;
                 const float nK = h.nK;
                 for (int r0 = h.r_first; r0 <= r_last; r0 += 32) {
@@ -493,6 +515,7 @@ __global__ void __launch_bounds__(kNormWarps * 32, 7)
                     if (cnt <= 0) continue;
                     float co[5];
                     poly_coeffs(A, B, nK, th, co);
+                    if (kind == K_POLY3) co[4] = 0.0f;   // (the deposits' polynomial)
                     const float2 v = ring_sum(co, d0h, 0.5f * rc.step, cnt, di);
                     total += cnt;
                     float err;
@@ -531,11 +554,13 @@ __global__ void __launch_bounds__(kNormWarps * 32, 7)
     if (lane == 0 && deposits) atomicAdd((unsigned long long *)(a.ctr + C_DEPOSITS), (unsigned long long)deposits);
 }
 
-constexpr int kGiantRings = 32;   // rings per claim of a giant disc
+constexpr int kGiantRings = 8;   // rings per claim of a giant disc
 constexpr int kGiantFold = 8;     // pixel pairs per plain FP32 partial
 
-// The giants, pixel by pixel: a warp takes 32 rings of a disc, one per lane
-// to build, and walks each with all lanes.
+// The giants, pixel by pixel: a warp takes kGiantRings rings of a disc, one per
+// lane to build, and walks each with all lanes (a ring has up to 4 nside
+// pixels, and few discs are giants: short claims spread them over the GPU; 0.34
+// ms, and 1.0 ms with claims of 32 rings).
 __global__ void __launch_bounds__(kNormWarps * 32)
     k_tile_norm_giant(const __grid_constant__ DiscArgs a, const __grid_constant__ TileArgs tg) {
     if (tg.ctl[0] != 2) return;
@@ -558,7 +583,7 @@ __global__ void __launch_bounds__(kNormWarps * 32)
         const Ext e = gen_ext(a, h);
         float s = 0.0f, c = 0.0f;
         Run g{};
-        if (ring <= h.r_last) {
+        if (lane < kGiantRings && ring <= h.r_last) {
             const RingT rc = ring_t(a, ring);
             int lo;
             g.cnt = max(0, tile_run<true>(a, h, rc, ring, lo, g.d0h, g.A, g.B));
@@ -566,7 +591,7 @@ __global__ void __launch_bounds__(kNormWarps * 32)
             g.A2 = antipode_term(h, rc);
         }
         __syncwarp();
-        for (int k = 0; k < 32; k++) {
+        for (int k = 0; k < kGiantRings; k++) {
             Run r{};
             r.cnt = __shfl_sync(0xffffffffu, g.cnt, k);
             if (r.cnt == 0) continue;
@@ -696,7 +721,8 @@ constexpr int kPairLanes = 8;   // lanes (strips at a time) per disc
 
 // MODE 0: the chunk's pairs, before S is known (for its mode; at least those
 // of mode 1, which leaves out discs with nothing to deposit); 1: pairs per
-// (tile, octave); 2: the pair list.
+// (tile, octave); 2: the pair list.  Bound by the latency of the slot atomics:
+// mode 2 takes 1.3 ms with four on their way, 2.7 ms one at a time.
 template <int MODE>
 __global__ void __launch_bounds__(256) k_tile_pairs(DiscArgs a, TileArgs tg) {
     if (MODE != 0 && tg.ctl[0] != 2) return;
@@ -705,7 +731,7 @@ __global__ void __launch_bounds__(256) k_tile_pairs(DiscArgs a, TileArgs tg) {
     const long long stride = (long long)gridDim.x * blockDim.x / kPairLanes;
     const int omax = MODE ? (int)a.ctr[C_OCT_MAX] : 0;
     const int NT = tg.nstrips * tg.ncol;
-    long long total = 0, list[3] = {0, 0, 0};
+    long long total = 0, list[kTileLists] = {};
     for (long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kPairLanes; q < nblk; q += stride) {
         TileHdr h = tg.hdr[q];
         int cls = 0;
@@ -724,18 +750,26 @@ __global__ void __launch_bounds__(256) k_tile_pairs(DiscArgs a, TileArgs tg) {
                 total += np;
                 continue;
             }
-            const int which = kind == K_POLY ? 0 : kind == K_GEN && nlo >= kFineNr ? 1 : 2, t0 = which * NT;
+            const int which = kind <= K_POLY ? kind : kind == K_GEN && nlo >= kFineNr ? 2 : 3, t0 = which * NT;
             if (MODE == 1) {
-                list[0] += which == 0 ? np : 0;
-                list[1] += which == 1 ? np : 0;
-                list[2] += which == 2 ? np : 0;
+#pragma unroll
+                for (int k = 0; k < kTileLists; k++) list[k] += which == k ? np : 0;
             }
-            for (int p = 0; p < 2; p++) {
-                const int ca = p ? c2 : c0, cb = p ? c3 : c1;
-                for (int c = ca; c <= cb; c++) {
-                    const int t = t0 + s * tg.ncol + c;
-                    const unsigned k = atomicAdd(tg.hist + ((size_t)t << kClsBits) + cls, 1u);
-                    if (MODE == 2) tg.list[tg.base[t] + k] = (unsigned)q;
+            // the columns of both ranges, four atomics on their way at a time
+            const int n0 = c1 - c0 + 1;
+            for (int i = 0; i < np; i += 4) {
+                unsigned k[4];
+                int t[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int c = i + u < n0 ? c0 + i + u : c2 + (i + u - n0);
+                    t[u] = t0 + s * tg.ncol + c;
+                    if (i + u < np) k[u] = atomicAdd(tg.hist + ((size_t)t[u] << kClsBits) + cls, 1u);
+                }
+                if (MODE == 2) {
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (i + u < np) tg.list[tg.base[t[u]] + k[u]] = (unsigned)q;
                 }
             }
         }
@@ -746,7 +780,7 @@ __global__ void __launch_bounds__(256) k_tile_pairs(DiscArgs a, TileArgs tg) {
     };
     if (MODE == 0) count(C_TILE_BOUND, total);
     if (MODE == 1)
-        for (int k = 0; k < 3; k++) count(C_TILE_PAIRS + k, list[k]);
+        for (int k = 0; k < kTileLists; k++) count(C_TILE_PAIRS + k, list[k]);
 }
 
 // Each tile's range of the pair list and its units: a warp per tile.
@@ -754,7 +788,7 @@ __global__ void __launch_bounds__(256) k_tile_plan(DiscArgs a, TileArgs tg) {
     if (tg.ctl[0] != 2) return;
     const int lane = threadIdx.x & 31;
     const int NT = tg.nstrips * tg.ncol;
-    const int nt = 3 * NT;
+    const int nt = kTileLists * NT;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     // enough units of each list to spread over the GPU, long enough to pay for
     // their flush
@@ -840,6 +874,8 @@ __device__ __forceinline__ Masks masks_of(const Piece &pc) {
 }
 
 // The deposits w F of group g (weights w, pair by pair) into the lane's row.
+// (Packed products with F = 0 in the lanes outside, where no lane covers the
+// group in part, took as long; and a weight outside the run may be infinite.)
 __device__ __forceinline__ void add_group(float2 (&acc)[kTileW / 2], int g, const Masks &mk,
                                           const float2 (&w)[kGroupPx / 2], float2 F) {
     const unsigned mw = mk.m[g * kGroupPx / 32] >> (g * kGroupPx % 32);
@@ -852,6 +888,7 @@ __device__ __forceinline__ void add_group(float2 (&acc)[kTileW / 2], int g, cons
 }
 
 // A piece of a polynomial disc.
+template <bool P3>
 __device__ __forceinline__ void add_poly(float2 (&acc)[kTileW / 2], const Piece &pc, const float c[5], float d0h,
                                          float steph, float2 F) {
     const Masks mk = masks_of(pc);
@@ -865,7 +902,7 @@ __device__ __forceinline__ void add_poly(float2 (&acc)[kTileW / 2], const Piece 
 #pragma unroll
         for (int k = 0; k < kGroupPx / 2; k++) {
             const float2 x = fma2(j, st2, d02);
-            w[k] = ex2_2(poly_exp2(c, mul2(x, x)));
+            w[k] = ex2_2(poly_exp2<P3>(c, mul2(x, x)));
             j = add2(j, two);
         }
         add_group(acc, g, mk, w, F);
@@ -995,8 +1032,13 @@ __device__ __forceinline__ float2 disc_F(const TileHdr &h, float2 phase) {
     return make_float2(h.p > phase.x ? h.Fn : h.F, h.p > phase.y ? h.Fn : h.F);
 }
 
-// Units of one list: 0 polynomial discs, 1 general discs on fine rings, 2 the
-// other general discs and the giants.
+// Units of one list: 0 and 1 polynomial discs (K_POLY3, K_POLY), 2 general
+// discs on fine rings, 3 the other general discs and the giants.  (Each list
+// has a kernel of its own: together they do not fit the instruction cache.)
+// Lists 0 to 2 take 19.5, 3.2 and 2.0 ms, the pixel kernel 0.8 ms.  Bound by
+// issue (72 % of the slots): per (disc, tile) about 580 instructions -- a ring's
+// chord test per lane, then 3.5 instructions a pixel (exponent, ex2, the
+// predicated product) over the groups that any lane covers.
 __device__ __forceinline__ bool claim_unit(const DiscArgs &a, const TileArgs &tg, int which, TileUnit &un) {
     long long u = 0;
     if ((threadIdx.x & 31) == 0) u = (long long)atomicAdd((unsigned long long *)(a.ctr + C_UNEXT + which), 1ull);
@@ -1006,15 +1048,16 @@ __device__ __forceinline__ bool claim_unit(const DiscArgs &a, const TileArgs &tg
     return true;
 }
 
-template <bool GEN>
+template <int LIST>
 __global__ void __launch_bounds__(kDepWarps * 32, kDepBlocks)
     k_tile_dep(const __grid_constant__ DiscArgs a, const __grid_constant__ TileArgs tg) {
     if (tg.ctl[0] != 2) return;
+    constexpr bool GEN = LIST == 2;
     __shared__ TileHdr sh[kDepWarps][2];
     __shared__ float tr[kDepWarps][32 * 33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     TileUnit un;
-    while (claim_unit(a, tg, GEN ? 1 : 0, un)) {
+    while (claim_unit(a, tg, LIST, un)) {
         const int strip = un.tile / tg.ncol, base = (un.tile - strip * tg.ncol) * kTileW;
         const int ring = min(strip * kTileR + 1 + lane, a.g.nrings);
         const bool own = strip * kTileR + 1 + lane <= a.g.nrings;
@@ -1042,13 +1085,13 @@ __global__ void __launch_bounds__(kDepWarps * 32, kDepBlocks)
                 if (h.flags & kFlagA2) r.A2 = antipode_term(h, rc);
                 e = gen_ext(a, h);
             } else {
-                poly_coeffs(r.A, r.B, h.nK, (h.flags & kFlagH1) ? 1 : 0, co);
+                poly_coeffs(r.A, r.B, h.nK, LIST == 1 && (h.flags & kFlagH1) ? 1 : 0, co);
             }
 #pragma unroll 1
             for (int p = 0;; p++) {
                 if (some) {
                     if constexpr (GEN) add_gen(acc, pc, e, r, F);
-                    else add_poly(acc, pc, co, r.d0h, r.steph, F);
+                    else add_poly<LIST == 0>(acc, pc, co, r.d0h, r.steph, F);
                 }
                 if (p == 1 || !second) break;
                 pc = Piece{0, 0, 0};
@@ -1093,7 +1136,7 @@ __global__ void __launch_bounds__(kGenWarps * 32)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float *const my = tile[w] + lane * kRow;
     TileUnit un;
-    while (claim_unit(a, tg, 2, un)) {
+    while (claim_unit(a, tg, 3, un)) {
         const int strip = un.tile / tg.ncol, base = (un.tile - strip * tg.ncol) * kTileW;
         const int ring = min(strip * kTileR + 1 + lane, a.g.nrings);
         const bool own = strip * kTileR + 1 + lane <= a.g.nrings;
@@ -1176,8 +1219,8 @@ cudaError_t launch_tile_norm(const DiscArgs &a, const TileArgs &tg, int num_sms,
 }
 
 cudaError_t launch_tile_deposits(const DiscArgs &a, const TileArgs &tg, int num_sms, cudaStream_t s) {
-    static const int occ = resident(k_tile_dep<false>, kDepWarps * 32), occg = resident(k_tile_dep<true>, kDepWarps * 32),
-                     occp = resident(k_tile_dep_px, kGenWarps * 32);
+    static const int occ0 = resident(k_tile_dep<0>, kDepWarps * 32), occ1 = resident(k_tile_dep<1>, kDepWarps * 32),
+                     occ2 = resident(k_tile_dep<2>, kDepWarps * 32), occp = resident(k_tile_dep_px, kGenWarps * 32);
     k_tile_fin<<<num_sms * 8, 256, 0, s>>>(a, tg);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -1187,9 +1230,11 @@ cudaError_t launch_tile_deposits(const DiscArgs &a, const TileArgs &tg, int num_
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     k_tile_pairs<2><<<num_sms * 8, 256, 0, s>>>(a, tg);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_tile_dep<false><<<num_sms * occ, kDepWarps * 32, 0, s>>>(a, tg);
+    k_tile_dep<0><<<num_sms * occ0, kDepWarps * 32, 0, s>>>(a, tg);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_tile_dep<true><<<num_sms * occg, kDepWarps * 32, 0, s>>>(a, tg);
+    k_tile_dep<1><<<num_sms * occ1, kDepWarps * 32, 0, s>>>(a, tg);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    k_tile_dep<2><<<num_sms * occ2, kDepWarps * 32, 0, s>>>(a, tg);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     k_tile_dep_px<<<num_sms * occp, kGenWarps * 32, 0, s>>>(a, tg);
     return cudaGetLastError();

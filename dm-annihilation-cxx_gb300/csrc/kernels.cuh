@@ -44,16 +44,17 @@ enum Ctr {
     C_SEG_MODE,        // the chunk's render: 0 per-disc kernels, 1 segments, 2 tiles
     // tiled render (disc_tile.cu)
     C_TILE_BOUND,      // (disc, tile) pairs, counted before the mode is known
-    C_TILE_PAIRS,      // the pairs of the three lists
-    C_TILE_PAIRS_LAST = C_TILE_PAIRS + 2,
+    C_TILE_PAIRS,      // the pairs of each list
+    C_TILE_PAIRS_LAST = C_TILE_PAIRS + 3,
     C_TILE_NEXT, C_GEN, C_GEN_NEXT,     // discs claimed; giant discs, parts of them claimed
     C_TILE_CURSOR,     // pair list slots handed out
-    C_UNITS, C_UNEXT = C_UNITS + 3,     // work units of the three lists, and claims
-    C_UNEXT_LAST = C_UNEXT + 2,
+    C_UNITS, C_UNEXT = C_UNITS + 4,     // work units of each list, and claims
+    C_UNEXT_LAST = C_UNEXT + 3,
     C_OCT_MAX,         // largest biased FP32 exponent of F
     C_COUNT
 };
 constexpr int kCtrChunkFirst = C_ADD_DISC;
+static_assert(C_COUNT * 8 <= 256, "the no-allocation render's layout holds 256 bytes of counters");
 
 struct Particles {
     const float *x, *y, *z, *m, *rho, *h;
@@ -157,6 +158,7 @@ struct SegArgs {
 constexpr int kTileR = 32, kTileW = 64;
 constexpr int kUnitMin = 32, kUnitMax = 512, kUnitTarget = 16384;
 constexpr int kTileClasses = 64;
+constexpr int kTileLists = 4;
 
 struct TileUnit {
     long long start;   // of its part of the pair list
@@ -181,9 +183,9 @@ struct TileArgs {
     const int *ctl;           // SegArgs::ctl: 2 when the chunk is rendered by tiles
     int nstrips, ncol;        // tiles of the map: strips of kTileR rings x columns
     unsigned *list;           // the pairs' discs, tile by tile
-    unsigned *hist;           // [3 tiles][kTileClasses]: pairs per octave, then list slots (a third per list)
-    long long *base;          // [3 tiles]: each tile's first list slot
-    TileUnit *units;          // [3][unit_cap]
+    unsigned *hist;           // [kTileLists][tiles][kTileClasses]: pairs per octave, then list slots
+    long long *base;          // [kTileLists][tiles]: each tile's first list slot
+    TileUnit *units;          // [kTileLists][unit_cap]
     long long unit_cap;
     double *disc_S;           // per block-class disc, as SegArgs
     long long *disc_px;
