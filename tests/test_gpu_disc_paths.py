@@ -17,6 +17,7 @@ import numpy as np
 import pytest
 
 import annmap
+import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -88,3 +89,30 @@ def test_plain_form(rend, nside, theta, radius, edge):
     grad, _ = rend.adjoint(parts, nside, G, precision=PLAIN)
     L = float(G @ rend.render(parts, nside, PLAIN))
     assert abs(grad[3, 0] - L) <= 1e-9 * L
+
+
+@pytest.fixture(scope="module")
+def vectors():
+    h = O.Healpix(128)
+    return np.array([h.pix2vec(p) for p in range(h.npix)])
+
+
+# The compensated adjoint of one disc in each pair of polynomial lengths that a
+# disc can have, by either kernel.  L = sum G map is linear in m, and its error
+# that of the weights (1e-5 of each, above) times G's range over G (at most 1)
+# and G's rounding: 1.1e-5.  G rises linearly along a tangent t, so the terms
+# (G - Gm) w e of the position's gradient are aligned: the weights' 1e-5 grows
+# by E|e_t||e| / E e_t^2 = 1.3 to 2e-5 with the tangent's own roundings, and G
+# and Gm, rounded to 6e-8 of 1.5, against 0.2 R: 5e-7 / R.
+@pytest.mark.parametrize("theta,radius", [(1.5, 0.03), (1.5, 0.1), (1.5, 0.2), (1.5, 0.5), (0.05, 0.1)])
+@pytest.mark.parametrize("edge", [64, 1 << 28])
+def test_adjoint_tiers(rend, vectors, theta, radius, edge):
+    nside, phi = 128, 2.0
+    rend.set_tuning(warp_max_pixels=edge, seg_min_deposits_log2=62)
+    parts = disc(theta, phi, radius)
+    t = np.array([math.cos(theta) * math.cos(phi), math.cos(theta) * math.sin(phi), -math.sin(theta)])
+    G = 1.0 + 0.5 * (vectors @ t)
+    got, _ = rend.adjoint(parts, nside, G, precision=COMP)
+    ref, _ = rend.adjoint(parts, nside, G, precision=PLAIN)
+    assert abs(got[3, 0] - ref[3, 0]) <= 1.1e-5 * abs(ref[3, 0])
+    assert np.linalg.norm(got[:3] - ref[:3]) <= (2e-5 + 5e-7 / radius) * np.linalg.norm(ref[:3])
