@@ -231,11 +231,45 @@ __device__ __forceinline__ void kahan(float &s, float &c, float v) {
     s = t;
 }
 
-// The sums of the disc particle whose header is staged.  Bound by issue (about
-// 150 instructions per pixel pair over both passes, most of them the division,
-// the square roots and Kahan's sums): with the series' lengths TX, TH (see
-// weight2x) read at run time instead, 1M particles at Nside 512 took 60.0 ms;
-// 56.4 with them.  The values, pixel by pixel, are the same bits.
+__device__ __forceinline__ void kahan2(float2 &s, float2 &c, float2 v) {
+    const float2 y = sub2(v, c);
+    const float2 t = add2(s, y);
+    c = sub2(sub2(t, s), y);
+    s = t;
+}
+
+// a / b and sqrt(a), correctly rounded, two at a time and without branches
+// (Markstein's corrections with exact FMA remainders: P. Markstein, IBM J. Res.
+// Dev. 34 (1990) 111).  a, b and the results normal, b above 2^-100; the results
+// equal __fdiv_rn's on 8e9 pairs with quotients of 2^-2 to 2^26 and
+// __fsqrt_rn's on every float of [2^-100, 2^31).  sqrt2_rn(0) is NaN.
+__device__ __forceinline__ float2 div2_rn(float2 a, float2 b) {
+    const float2 nb = mul2(b, f2(-1.0f));
+    float2 y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(b.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(b.y));
+    y = fma2(y, fma2(nb, y, f2(1.0f)), y);
+    const float2 q = mul2(a, y);
+    return fma2(fma2(nb, q, a), y, q);
+}
+__device__ __forceinline__ float2 sqrt2_rn(float2 a) {
+    float2 y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(a.x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(a.y));
+    float2 g = mul2(a, y), h = mul2(y, f2(-0.5f));
+    const float2 r = fma2(g, h, f2(0.5f));
+    g = fma2(g, r, g);
+    h = fma2(h, r, h);
+    return fma2(fma2(g, g, mul2(a, f2(-1.0f))), h, g);
+}
+
+// The sums of the disc particle whose header is staged.  Bound by issue (78 %
+// of the slots), so by the instructions per pixel pair: with the series'
+// lengths TX, TH (see weight2x) read at run time 1M particles at Nside 512 took
+// 60.0 ms, with them fixed 56.4, and 49.1 with the second pass in packed
+// arithmetic and its division and square roots free of branches.  Each step
+// kept every value, bit by bit: the gradient of the observer's position is a
+// sum of cancelling terms.
 template <int G, int RCH, int TX, int TH>
 __device__ void adjc_disc(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long long q, AdjSums *sums) {
     using Gp = Grp<G>;
@@ -297,7 +331,8 @@ __device__ void adjc_disc(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long long q,
     const float gm = gq.x;   // sum G w / S rounded
 
     // pass 2: V_theta, V_phi, T with q = (G - Gm) w
-    float vts = 0.0f, vtc = 0.0f, vps = 0.0f, vpc = 0.0f, ts = 0.0f, tc = 0.0f;
+    float2 vs = f2(0.0f), vc = f2(0.0f);
+    float ts = 0.0f, tc = 0.0f;
     for (int c = 0; c < nchunk; c++) {
         const int r0 = r_first + c * RCH;
         const int n = min(RCH, r_last - r0 + 1);
@@ -312,31 +347,39 @@ __device__ void adjc_disc(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long long q,
             const float2 w = weight2x<TX, TH>(e, r, make_float2(jf, jf + (float)off), sn, h, g);
             const AdjRing ar = sm.aring[ring];
             const int pix = r.pix0 + j;
-            float vt = 0.0f, vp = 0.0f, tt = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                if (k == 1 && !second) break;
-                const float wk = k ? w.y : w.x, snk = k ? sn.y : sn.x, hk = k ? h.y : h.x,
-                            gk = k ? g.y : g.x;
-                const float q = (g32[k ? pix + off : pix] - gm) * wk;
-                // alpha / sin(alpha); 0 at the antipode, where the tangent is undefined
-                const float om = 1.0f - hk;
-                const float af = hk > 1e-30f ? (om > 1e-7f ? sqrtf(gk / (hk * om)) : 0.0f) : 1.0f;
-                const float s2 = snk * snk;
-                const float eth = fmaf(-ar.cr, s2, ar.sr);
-                const float eph = ar.st2 * snk * sqrtf(fmaxf(1.0f - s2, 0.0f));
-                const float qa = q * af;
-                vt = fmaf(qa, eth, vt);
-                vp = fmaf(qa, eph, vp);
-                tt = fmaf(q, 4.0f * gk, tt);
+            const float2 q = mul2(sub2(make_float2(g32[pix], second ? g32[pix + off] : 0.0f), f2(gm)), w);
+            // alpha / sin(alpha); 0 at the antipode, where the tangent is undefined
+            const float2 om = sub2(f2(1.0f), h);
+            float2 af = sqrt2_rn(div2_rn(g, mul2(h, om)));
+            if (TH < 0) {
+                if (!(om.x > 1e-7f)) af.x = 0.0f;
+                if (!(om.y > 1e-7f)) af.y = 0.0f;
             }
-            kahan(vts, vtc, vt);
-            kahan(vps, vpc, vp);
+            if (!(h.x > 1e-30f)) af.x = 1.0f;
+            if (!(h.y > 1e-30f)) af.y = 1.0f;
+            const float2 s2 = mul2(sn, sn);
+            const float2 c2 = sub2(f2(1.0f), s2);
+            float2 cs = sqrt2_rn(c2);
+            if (TX < 0) {
+                if (!(c2.x > 0.0f)) cs.x = 0.0f;
+                if (!(c2.y > 0.0f)) cs.y = 0.0f;
+            }
+            const float2 eth = fma2(f2(-ar.cr), s2, f2(ar.sr));
+            const float2 eph = mul2(mul2(f2(ar.st2), sn), cs);
+            const float2 qa = mul2(q, af), g4 = mul2(f2(4.0f), g);
+            float2 v = make_float2(__fmul_rn(qa.x, eth.x), __fmul_rn(qa.x, eph.x));
+            float tt = __fmul_rn(q.x, g4.x);
+            if (second) {   // (beyond the run its values may be infinite or NaN)
+                v.x = fmaf(qa.y, eth.y, v.x);
+                v.y = fmaf(qa.y, eph.y, v.y);
+                tt = fmaf(q.y, g4.y, tt);
+            }
+            kahan2(vs, vc, v);
             kahan(ts, tc, tt);
         });
         Gp::sync();
     }
-    float2 vt = make_float2(vts, -vtc), vp = make_float2(vps, -vpc), tt = make_float2(ts, -tc);
+    float2 vt = make_float2(vs.x, -vc.x), vp = make_float2(vs.y, -vc.y), tt = make_float2(ts, -tc);
     group_sum_ff<G>(vt, sm.red[2]);
     group_sum_ff<G>(vp, sm.red[3]);
     group_sum_ff<G>(tt, sm.red[4]);

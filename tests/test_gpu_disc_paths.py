@@ -104,7 +104,8 @@ def vectors():
 # (G - Gm) w e of the position's gradient are aligned: the weights' 1e-5 grows
 # by E|e_t||e| / E e_t^2 = 1.3 to 2e-5 with the tangent's own roundings, and G
 # and Gm, rounded to 6e-8 of 1.5, against 0.2 R: 5e-7 / R.
-@pytest.mark.parametrize("theta,radius", [(1.5, 0.03), (1.5, 0.1), (1.5, 0.2), (1.5, 0.5), (0.05, 0.1)])
+@pytest.mark.parametrize("theta,radius", [(1.5, 0.03), (1.5, 0.1), (1.5, 0.2), (1.5, 0.5), (0.05, 0.1),
+                                          (1.2, 2.5)])
 @pytest.mark.parametrize("edge", [64, 1 << 28])
 def test_adjoint_tiers(rend, vectors, theta, radius, edge):
     nside, phi = 128, 2.0
