@@ -12,6 +12,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/dmann.h"
@@ -258,6 +259,36 @@ bool is_device_ptr(const void *p) {
         return false;
     }
     return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
+}
+
+// Touches the pages of a pageable output buffer (its bytes keep their values)
+// from several threads while the GPU still renders. A fresh allocation has no
+// pages yet; the copy faulted them in one by one: 21 of 26 ms of the last call
+// of a streamed map at Nside 512 (25 MB), which takes 4 ms into mapped pages.
+void fault_in(void *buf, size_t bytes) {
+    constexpr size_t kPage = 4096, kPerThread = (size_t)2 << 20;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, buf) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (bytes < 2 * kPerThread || at.type != cudaMemoryTypeUnregistered) return;
+    const size_t hw = std::max(2u, std::thread::hardware_concurrency());
+    const size_t nt = std::min({(size_t)8, hw / 2, bytes / kPerThread}), part = bytes / nt;
+    auto touch = [=](size_t k) {
+        volatile char *const c = (volatile char *)buf;
+        const size_t end = k + 1 < nt ? (k + 1) * part : bytes;
+        for (size_t i = k * part; i < end; i += kPage) c[i] = c[i];
+        c[end - 1] = c[end - 1];
+    };
+    std::thread th[8];
+    size_t n = 0;
+    try {
+        for (; n + 1 < nt; n++) th[n] = std::thread(touch, n + 1);
+        touch(0);
+    } catch (...) {   // no thread to be had: the copy faults the rest in
+    }
+    for (size_t k = 0; k < n; k++) th[k].join();
 }
 
 Hpx make_hpx(int nside) {
@@ -1034,6 +1065,7 @@ dmann_status dmann_map_end(dmann_ctx *ctx, double *map_out, int accumulate) {
     ctx->stats_pending = true;
     ctx->in_map = false;
     if (!map_dev) {
+        fault_in(map_out, 8 * P);
         CK(cudaMemcpyAsync(map_out, dmap, 8 * P, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
     }

@@ -117,3 +117,21 @@ def test_adjoint_tiers(rend, vectors, theta, radius, edge):
     ref, _ = rend.adjoint(parts, nside, G, precision=PLAIN)
     assert abs(got[3, 0] - ref[3, 0]) <= 1.1e-5 * abs(ref[3, 0])
     assert np.linalg.norm(got[:3] - ref[:3]) <= (2e-5 + 5e-7 / radius) * np.linalg.norm(ref[:3])
+
+
+# Host maps on either side of the size from which their pages are touched ahead
+# of the copy (4 MB: Nside 209), fresh and at an odd offset in a larger buffer
+# whose neighbours stay as they are; the sums are FP64 in an order of their own.
+@pytest.mark.parametrize("nside", [64, 209, 300])
+def test_host_map(rend, nside):
+    torch = pytest.importorskip("torch")
+    rend.set_tuning(seg_min_deposits_log2=62)
+    parts = disc(1.0, 2.0, 0.7)
+    npix = 12 * nside * nside
+    dev = torch.zeros(npix, dtype=torch.float64, device="cuda")
+    rend.render({k: torch.from_numpy(v).cuda() for k, v in parts.items()}, nside, PLAIN, out=dev)
+    buf = np.full(npix + 2, -7.0)
+    rend.render(parts, nside, PLAIN, out=buf[1:-1])
+    assert buf[0] == -7.0 and buf[-1] == -7.0
+    for got in (buf[1:-1], rend.render(parts, nside, PLAIN)):
+        np.testing.assert_allclose(got, dev.cpu().numpy(), rtol=1e-12, atol=0)
