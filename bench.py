@@ -152,20 +152,10 @@ def measured_peaks():
     return 6800.0, "fallback"
 
 
-def profile_traffic():
-    """Per-deposit DRAM bytes of the deposit kernel from the committed ncu summary."""
-    p = os.path.join(REPO, "profiles", "disc_seg_traffic.json")
-    if os.path.exists(p):
-        with open(p) as f:
-            return json.load(f)
-    return None
-
-
 def measure_l2_red(device, plane_floats):
     """Live L2 reduction rates (operations/s) of the library's own sweep
-    microbenchmark: FP32 red (the compensated form's deposit) over an array
-    the size of the FP32 deposit plane (the footprint the deposits land
-    in), and for reference FP32 and FP64 red over 400 MB."""
+    microbenchmark: FP32 red over an array the size of an FP32 map, and
+    FP32 and FP64 red over 400 MB."""
     import ctypes as C
     from annmap import _lib
     L = _lib.load()
@@ -180,42 +170,41 @@ def measure_l2_red(device, plane_floats):
     return out
 
 
-FP32_FLOPS_PER_WEIGHT = 12   # x (FMA), y = x^2, 4 Horner FMAs, the sum: 2 + 1 + 8 + 1
+# x (FMA), y = x^2, 4 Horner FMAs, the sum or the deposit (FMA); the ex2 is apart
+FP32_FLOPS_PER_DEPOSIT = 2 + 1 + 8 + 2
 
 
 def roofline(device, deposits, pass1_ms, pass2_ms, npix):
-    """The deposit pass's roofline on its binding resource, the L2 reduction
-    units: each algorithmic deposit is one FP32 reduction (4 B) into the
-    map's FP32 plane, against the library's live red.global.add.f32 sweep.
-    Beside it the same bytes against measured HBM, and pass 1 (weight sums:
-    FP32 arithmetic, no memory traffic to speak of) against the nominal FP32
-    rate of the FMA pipes."""
+    """The deposit pass's roofline on its binding resource, FP32 issue: each
+    algorithmic deposit is a weight and a multiply-add into a register
+    (tiles of the map are held in registers, so only a pixel per tile and
+    work unit reaches memory), against the nominal FP32 rate of the FMA
+    pipes. Beside it what the same deposits would need as one FP32 reduction
+    each, against the library's live red.global.add.f32 sweep and against
+    measured HBM; and pass 1 (weight sums by quadrature: its operations do
+    not grow with the deposits) as deposits normalised per second."""
     l2 = measure_l2_red(device, npix)
     hbm, hbm_src = measured_peaks()
-    red_bytes = 4.0 * deposits
     s2, s1 = pass2_ms / 1e3, pass1_ms / 1e3
-    achieved = red_bytes / s2 / 1e9
-    peak = (l2["red_f32"] or 0.0) * 4.0 / 1e9
-    traffic = profile_traffic()
-    nominal_fp32 = 152 * 128 * 2 * 2.07e9 / 1e12
-    p1_tflops = deposits * FP32_FLOPS_PER_WEIGHT / s1 / 1e12
-    return {"bound": "l2_red", "kernel": "k_seg_dep (deposit segments)", "achieved": achieved,
-            "peak": peak, "unit": "GB/s", "frac": achieved / peak if peak else None,
-            "peak_source": (f"measured here: red.global.add.f32 sweep over the deposit plane's "
-                            f"{l2['plane_bytes'] / 1e6:.0f} MB ({l2['red_f32']:.3e} reductions/s)")
-            if l2["red_f32"] else "unavailable",
-            "traffic": (traffic["dram_bytes_per_deposit"] * deposits) if traffic else None,
-            "traffic_source": traffic.get("capture") if traffic else None,
-            "algorithmic_bytes": red_bytes,
-            "basis": "4 B FP32 reduction per algorithmic deposit / deposit-pass time (CUDA events)",
-            "hbm": {"achieved": achieved, "peak": hbm, "frac": achieved / hbm,
+    achieved = deposits * FP32_FLOPS_PER_DEPOSIT / s2 / 1e12
+    peak = 152 * 128 * 2 * 2.07e9 / 1e12
+    red_bytes = 4.0 * deposits
+    red_gbs = red_bytes / s2 / 1e9
+    red_peak = (l2["red_f32"] or 0.0) * 4.0 / 1e9
+    return {"bound": "fp32_issue", "kernel": "k_tile_dep (pair list and tile deposits)",
+            "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
+            "peak_source": "nominal: 152 SMs x 128 FP32 lanes x FMA x 2.07 GHz",
+            "traffic": None, "algorithmic_bytes": red_bytes,
+            "basis": f"{FP32_FLOPS_PER_DEPOSIT} FP32 operations per algorithmic deposit / deposit-pass time (CUDA events)",
+            "as_reductions": {"achieved": red_gbs, "peak": red_peak, "unit": "GB/s",
+                              "frac": red_gbs / red_peak if red_peak else None,
+                              "peak_source": (f"measured here: red.global.add.f32 sweep over "
+                                              f"{l2['plane_bytes'] / 1e6:.0f} MB ({l2['red_f32']:.3e} reductions/s)")
+                              if l2["red_f32"] else "unavailable"},
+            "hbm": {"achieved": red_gbs, "peak": hbm, "frac": red_gbs / hbm,
                     "peak_source": hbm_src + " (MEASURED_PEAKS hbm_gbs)"},
             "sweeps_400mb": {"red_f32": l2["red_f32_400mb"], "red_f64": l2["red_f64_400mb"]},
-            "pass1": {"kernel": "k_seg_norm (weight sums)", "ms": pass1_ms, "weights_per_s": deposits / s1,
-                      "fp32_flops_per_weight": FP32_FLOPS_PER_WEIGHT, "achieved_tflops": p1_tflops,
-                      "peak_tflops": nominal_fp32,
-                      "peak_source": "nominal: 152 SMs x 128 FP32 lanes x FMA x 2.07 GHz",
-                      "frac": p1_tflops / nominal_fp32}}
+            "pass1": {"kernel": "k_tile_norm (weight sums)", "ms": pass1_ms, "deposits_per_s": deposits / s1}}
 
 
 def rel_err(got, ref):
