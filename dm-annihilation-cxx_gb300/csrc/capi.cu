@@ -748,21 +748,6 @@ size_t seg_capacity(size_t n) {
     return std::min<size_t>(4 * (n > 0 ? n : 1) + ((size_t)1 << 20), (size_t)0x7fffffff);
 }
 
-// Pair list slots of the tiled render: every disc in every tile where that
-// is little (then no chunk can exceed it), else 96 per particle and 2^24 (a
-// disc of the 16M set at Nside 2048 touches 33 tiles, one of the 134M set at
-// Nside 4096 about 55; chunks with more pairs are segmented).
-size_t tile_pairs_bound(size_t n, int nside) {
-    return (n > 0 ? n : 1) * (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
-}
-size_t tile_capacity(size_t n, int nside) {
-    return std::min(tile_pairs_bound(n, nside), 96 * n + ((size_t)1 << 24));
-}
-size_t tile_unit_capacity(size_t n, int nside) {
-    return tile_capacity(n, nside) / kUnitMax + 2 * (size_t)kUnitTarget +
-           (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
-}
-
 // The buffers of the two large-chunk renders for chunks of n particles at
 // one Nside: grown when grow is set (a failed allocation is not an error: the
 // chunk takes a render that does without), else only looked at, as under
@@ -802,7 +787,6 @@ bool may_be_large(size_t n, int nside, const dmann_tuning &tu) {
     const int lg = tu.seg_min_deposits_log2 > 0 ? tu.seg_min_deposits_log2 : 28;
     return (double)n * 12.0 * nside * nside >= std::ldexp(1.0, lg);
 }
-bool tile_always_fits(size_t n, int nside) { return tile_capacity(n, nside) == tile_pairs_bound(n, nside); }
 
 bool reserve_large(dmann_ctx *ctx, size_t n, int nside, const dmann_tuning &tu) {
     if (!may_be_large(n, nside, tu)) return true;
@@ -828,8 +812,8 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     const int nside = ctx->g.nside;
     if (!da.chdr || !may_be_large(N, nside, tu)) return DMANN_OK;
     Work &w = *ctx->w;
-    const bool tile = have_tile(ctx, N, nside, grow);
-    const bool seg = !(tile && tile_always_fits(N, nside)) && have_seg(ctx, N, nside, grow);
+    const bool have_t = have_tile(ctx, N, nside, grow), fits = tile_always_fits(N, nside);
+    const auto [tile, seg, count] = plan_large(have_t, fits, !(have_t && fits) && have_seg(ctx, N, nside, grow));
     if (!tile && !seg) return DMANN_OK;
     cudaStream_t s = ctx->stream;
     const int bt = tu.block_threads == 128 ? 128 : 256;
@@ -870,7 +854,7 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
         CK(cudaMemsetAsync(w.tile_hist.p, 0, kTileLists * (size_t)tg.nstrips * tg.ncol * kTileClasses * sizeof(unsigned), s));
     CK(launch_hdr(da, ctx->num_sms, s));
     CK(launch_seg_count(da, sg, bt, ctx->num_sms, s));
-    if (tile) CK(launch_tile_hdr(da, tg, seg, ctx->num_sms, s));
+    if (tile) CK(launch_tile_hdr(da, tg, count, ctx->num_sms, s));
     CK(launch_seg_decide(da, sg, s));
     ctx->launches += 8;   // prep, scan, scatter, headers, counts, mode, block kernel, warp class
     if (seg) CK(launch_seg_norm(da, sg, bt, ctx->num_sms, tu.blocks_per_sm, s));
@@ -878,7 +862,7 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     if (timed) CK(cudaEventRecord(ctx->evp1, s));
     if (tile) {
         CK(launch_tile_deposits(da, tg, ctx->num_sms, s));
-        ctx->launches += 11 + (seg ? 1 : 0);
+        ctx->launches += 11 + (count ? 1 : 0);
     }
     if (seg) {
         w.plane_clean = false;

@@ -430,17 +430,10 @@ __global__ void __launch_bounds__(256) k_seg_count(DiscArgs a, SegArgs sg) {
         atomicAdd((unsigned long long *)(a.ctr + C_SEG_EST), (unsigned long long)est_sum);
 }
 
-// The chunk's mode.  From min_est estimated deposits on it is rendered by
-// tiles where the pair list holds its pairs, else in segments where the item
-// buffers hold its items, else (and below min_est) by the per-disc kernels
-// with FP64 deposits.
+// The chunk's mode (large_mode in tile_plan.h).
 __global__ void k_seg_decide(DiscArgs a, SegArgs sg) {
-    int mode = 0;
-    if (a.ctr[C_SEG_EST] >= sg.min_est && a.ctr[C_ADD_BLOCK] > 0) {
-        const long long items = a.ctr[C_SEG_ITEMS];
-        if (sg.pair_cap > 0 && a.ctr[C_TILE_BOUND] <= sg.pair_cap) mode = 2;
-        else if (items > 0 && items <= sg.cap) mode = 1;
-    }
+    const int mode = large_mode(a.ctr[C_SEG_EST], sg.min_est, a.ctr[C_ADD_BLOCK], a.ctr[C_TILE_BOUND], sg.pair_cap,
+                                a.ctr[C_SEG_ITEMS], sg.cap);
     sg.ctl[0] = mode;
     a.ctr[C_SEG_MODE] = mode;
 }

@@ -1201,10 +1201,10 @@ int resident(K k, int threads) {
 
 }  // namespace
 
-cudaError_t launch_tile_hdr(const DiscArgs &a, const TileArgs &tg, bool total, int num_sms, cudaStream_t s) {
+cudaError_t launch_tile_hdr(const DiscArgs &a, const TileArgs &tg, bool count, int num_sms, cudaStream_t s) {
     k_tile_hdr<<<num_sms * 8, 256, 0, s>>>(a, tg);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || !total) return e;
+    if (e != cudaSuccess || !count) return e;
     k_tile_pairs<0><<<num_sms * 8, 256, 0, s>>>(a, tg);
     return cudaGetLastError();
 }

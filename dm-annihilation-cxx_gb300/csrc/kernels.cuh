@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include "common.cuh"
 #include "seg_plan.h"
+#include "tile_plan.h"
 
 namespace dmann {
 
@@ -152,14 +153,7 @@ struct SegArgs {
     float *plane;             // FP32 deposit plane, npix floats, zero between segments
 };
 
-// Tiled render of the block-class discs (disc_tile.cu): a tile is kTileR rings
-// by kTileW in-ring pixel indices, a unit up to kUnitMax discs of its list
-// (fewer while the chunk has less than kUnitTarget units of more than kUnitMin).
-constexpr int kTileR = 32, kTileW = 64;
-constexpr int kUnitMin = 32, kUnitMax = 512, kUnitTarget = 16384;
-constexpr int kTileClasses = 64;
-constexpr int kTileLists = 4;
-
+// Tiled render of the block-class discs (disc_tile.cu; its sizes are in tile_plan.h).
 struct TileUnit {
     long long start;   // of its part of the pair list
     int len, tile;
@@ -191,9 +185,6 @@ struct TileArgs {
     long long *disc_px;
     int *gen;                 // queue slots of the giant discs (C_GEN of them)
 };
-
-inline int tile_strips(int nside) { return (4 * nside - 1 + kTileR - 1) / kTileR; }
-inline int tile_cols(int nside) { return (4 * nside + kTileW - 1) / kTileW; }
 
 // prep.cu
 cudaError_t launch_prep(const PrepArgs &a, cudaStream_t s);
@@ -237,10 +228,10 @@ cudaError_t launch_seg_norm(const DiscArgs &a, const SegArgs &sg, int block_thre
 cudaError_t launch_seg_sort(const DiscArgs &a, const SegArgs &sg, int num_sms, cudaStream_t s);
 cudaError_t launch_seg_deposits(const DiscArgs &a, const SegArgs &sg, int block_threads, int num_sms,
                                 int blocks_per_sm, int npix, cudaStream_t s);
-// disc_tile.cu, in stream order, each returning at once unless the chunk's
-// mode is 2: the tile headers and (total) the pair count, before the mode is
-// decided; the weight sums; F, the pair list and the deposits.
-cudaError_t launch_tile_hdr(const DiscArgs &a, const TileArgs &tg, bool total, int num_sms, cudaStream_t s);
+// disc_tile.cu, in stream order: the tile headers and (count) the chunk's
+// pairs, before the mode is decided; then, returning at once unless the mode
+// is 2, the weight sums; F, the pair list and the deposits.
+cudaError_t launch_tile_hdr(const DiscArgs &a, const TileArgs &tg, bool count, int num_sms, cudaStream_t s);
 cudaError_t launch_tile_norm(const DiscArgs &a, const TileArgs &tg, int num_sms, cudaStream_t s);
 cudaError_t launch_tile_deposits(const DiscArgs &a, const TileArgs &tg, int num_sms, cudaStream_t s);
 // disc_comp.cu: the compensated block kernel alone (headers built)

@@ -1,0 +1,65 @@
+// tile_plan.h -- sizes of the tiled render's buffers (disc_tile.cu) and the
+// choice between the renders of a large chunk, in a header a host compiler
+// also takes, so both are unit-tested on the CPU.
+#pragma once
+#include <algorithm>
+#include <cstddef>
+
+#include "seg_plan.h"
+
+namespace dmann {
+
+// A tile is kTileR rings by kTileW in-ring pixel indices, a unit up to
+// kUnitMax discs of its list (fewer while the chunk has less than kUnitTarget
+// units of more than kUnitMin).
+constexpr int kTileR = 32, kTileW = 64;
+constexpr int kUnitMin = 32, kUnitMax = 512, kUnitTarget = 16384;
+constexpr int kTileClasses = 64;
+constexpr int kTileLists = 4;
+
+inline int tile_strips(int nside) { return (4 * nside - 1 + kTileR - 1) / kTileR; }
+inline int tile_cols(int nside) { return (4 * nside + kTileW - 1) / kTileW; }
+
+// Every disc of a chunk in every tile.
+inline size_t tile_pairs_bound(size_t n, int nside) {
+    return (n > 0 ? n : 1) * (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
+}
+// Pair list slots of the tiled render: every disc in every tile where that
+// is little (then no chunk can exceed it), else 96 per particle and 2^24 (a
+// disc of the 16M set at Nside 2048 touches 33 tiles, one of the 134M set at
+// Nside 4096 about 55; chunks with more pairs are segmented).
+inline size_t tile_capacity(size_t n, int nside) {
+    return std::min(tile_pairs_bound(n, nside), 96 * n + ((size_t)1 << 24));
+}
+inline size_t tile_unit_capacity(size_t n, int nside) {
+    return tile_capacity(n, nside) / kUnitMax + 2 * (size_t)kUnitTarget +
+           (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
+}
+inline bool tile_always_fits(size_t n, int nside) { return tile_capacity(n, nside) == tile_pairs_bound(n, nside); }
+
+// The renders launched for a chunk that may be large, from the buffers there
+// are: the segments are of use where the pair list can overflow, and there the
+// chunk's pairs are counted whether or not there are segments to take it -- the
+// pair list's kernels write as many slots as there are pairs.
+struct LargePlan {
+    bool tile, seg;
+    bool count;   // k_tile_pairs<0> before the mode is decided
+};
+inline LargePlan plan_large(bool have_tile, bool always_fits, bool have_seg) {
+    const bool sure = have_tile && always_fits;
+    return LargePlan{have_tile, have_seg && !sure, have_tile && !sure};
+}
+
+// A chunk's mode (k_seg_decide): 2 tiles, 1 segments, 0 per-disc kernels.
+// From min_est estimated deposits on it is rendered by tiles where the pair
+// list (pair_cap slots; 0: none) holds its pairs (0 when they need no count),
+// else in segments where the item buffers (item_cap; 0: none) hold its items,
+// else (and below min_est) by the per-disc kernels with FP64 deposits.
+DMANN_HD inline int large_mode(long long est, long long min_est, long long blocks, long long pairs,
+                               long long pair_cap, long long items, long long item_cap) {
+    if (est < min_est || blocks <= 0) return 0;
+    if (pair_cap > 0 && pairs <= pair_cap) return 2;
+    return items > 0 && items <= item_cap ? 1 : 0;
+}
+
+}  // namespace dmann

@@ -1,0 +1,46 @@
+"""The choice between the renders of a large chunk (csrc/tile_plan.h, the
+functions capi.cu and k_seg_decide use), built for the host: a chunk is
+rendered by tiles only when its (disc, tile) pairs are known to fit the pair
+list, whatever other buffers there are."""
+import ctypes as C
+import itertools
+import os
+import subprocess
+
+import pytest
+
+REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(REPO, "dm-annihilation-cxx_gb300", "csrc")
+TILE, SEG, COUNT = 1, 2, 4
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("plan") / "libtileplan.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", CSRC,
+                    os.path.join(REPO, "tests", "cpp", "tile_plan_shim.cpp"), "-o", so], check=True)
+    d = C.CDLL(so)
+    for f in (d.pairs_bound, d.capacity):
+        f.restype, f.argtypes = C.c_longlong, [C.c_longlong, C.c_int]
+    d.always_fits.argtypes = [C.c_longlong, C.c_int]
+    d.mode.argtypes = [C.c_longlong] * 7
+    return d
+
+
+def chunk_mode(lib, n, nside, have_tile, have_seg, pairs, items):
+    """The mode that a chunk's launches and the device's decision come to."""
+    p = lib.plan(have_tile, lib.always_fits(n, nside), have_seg)
+    return lib.mode(1 << 40, 1 << 28, n, pairs if p & COUNT else 0, lib.capacity(n, nside) if p & TILE else 0,
+                    items if p & SEG else 0, 4 * n + (1 << 20) if p & SEG else 0)
+
+
+# a chunk whose pairs always fit, and two that can overflow
+@pytest.mark.parametrize("n,nside", [(1000, 64), (10000, 1024), (1 << 20, 4096)])
+def test_no_chunk_overflows_the_pair_list(lib, n, nside):
+    bound, cap = lib.pairs_bound(n, nside), lib.capacity(n, nside)
+    for tile, seg, pairs in itertools.product((0, 1), (0, 1), (1, cap, min(cap + 1, bound), bound)):
+        mode = chunk_mode(lib, n, nside, tile, seg, pairs, n)
+        if tile and pairs <= cap:
+            assert mode == 2
+        else:
+            assert mode == (1 if seg else 0), (tile, seg, pairs, cap)
