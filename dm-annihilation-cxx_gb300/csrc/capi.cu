@@ -838,6 +838,7 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     sg.plane = (float *)w.plane32.p;
     TileArgs tg{};
     tg.ctl = sg.ctl;
+    tg.flux_sum = (const double *)w.fsum.p;
     tg.nstrips = tile_strips(nside);
     tg.ncol = tile_cols(nside);
     tg.list = (unsigned *)w.tile_list.p;

@@ -59,10 +59,19 @@ enum Kind {
     K_POLY3 = 0,   // the ring's exponent polynomial without its y^4 term
     K_POLY = 1,    // the ring's exponent polynomial
     K_GEN = 2,     // run-time series per value
-    K_GIANT = 3    // the same; radius beyond kGiantR, which may reach the kink at the antipode
+    K_GIANT = 3    // the same, summed pixel by pixel and deposited in two floats: radius beyond
+                   // kGiantR (which may reach the kink at the antipode), or a share of the map's flux
 };
 constexpr int kKindMask = 3, kFlagH1 = 4, kFlagAll = 8, kFlagFast = 16, kFlagA2 = 32;
 constexpr double kGiantR = 2.2;
+
+// Discs with 1 / kShare and more of the flux kept so far are giants too.  The
+// quadrature's sum of one disc scatters by 5e-9 (up to 2e-8: a few thousand nodes
+// instead of the pixels, each exponent rounded to FP32), so the rest of a map is
+// off by 5e-9 / sqrt(kShare) = 3e-10 of its flux at most, few discs or many.  A
+// giant's own flux is off by 1e-12.  (kShareMax: with fluxes of both signs the
+// sum of flux bounds nothing.)
+constexpr int kShare = 256, kShareMax = 1024;
 
 // The y^4 term is at most 2.7e-8 in the exponent of 2 for half azimuth offsets
 // x below 0.1 rad (y = x^2) and the three-term asin^2 tier (h < 4e-3): a ninth
@@ -450,6 +459,9 @@ __global__ void __launch_bounds__(256) k_tile_hdr(DiscArgs a, TileArgs tg) {
             kind = c.ext.tier_h == 0 && sinf((float)c.hdr.R) < kPoly3Sin * c.ch.sth0 ? K_POLY3 : K_POLY;
         else
             kind = c.hdr.R < kGiantR ? K_GEN : K_GIANT;
+        if (kind != K_GIANT && c.hdr.flux != 0.0 && fabs(c.hdr.flux) * kShare >= fabs(*tg.flux_sum) &&
+            atomicAdd(tg.ctl + 2, 1) < kShareMax)
+            kind = K_GIANT;
         t.flags = kind | (c.ext.tier_h >= 1 ? kFlagH1 : 0) | (c.hdr.allsky ? kFlagAll : 0) |
                   (c.ch.fast ? kFlagFast : 0) | (c.ext.tier_h == 2 ? kFlagA2 : 0);
         tg.hdr[q] = t;
@@ -562,7 +574,6 @@ __global__ void __launch_bounds__(kNormWarps * 32, 7)
 }
 
 constexpr int kGiantRings = 8;   // rings per claim of a giant disc
-constexpr int kGiantFold = 8;     // pixel pairs per plain FP32 partial
 
 // The giants, pixel by pixel: a warp takes kGiantRings rings of a disc, one per
 // lane to build, and walks each with all lanes (a ring has up to 4 nside
@@ -588,7 +599,8 @@ __global__ void __launch_bounds__(kNormWarps * 32)
         __syncwarp();
         const int ring = h.r_first + (int)(t % parts) * kGiantRings + lane;
         const Ext e = gen_ext(a, h);
-        float s = 0.0f, c = 0.0f;
+        // each rounding of the sums kept: they start at 1, above every weight
+        float2 ks = f2(1.0f), kc = f2(0.0f);
         Run g{};
         if (lane < kGiantRings && ring <= h.r_last) {
             const RingT rc = ring_t(a, ring);
@@ -607,25 +619,17 @@ __global__ void __launch_bounds__(kNormWarps * 32)
             r.A2 = __shfl_sync(0xffffffffu, g.A2, k);
             r.d0h = __shfl_sync(0xffffffffu, g.d0h, k);
             r.steph = __shfl_sync(0xffffffffu, g.steph, k);
-            float2 part = f2(0.0f);
-            int np = 0;
             for (int j = lane; j < r.cnt; j += 64) {
                 const float jf = (float)j;
                 float2 w = weight2<-1, -1>(e, r, make_float2(jf, jf + 32.0f));
                 if (j + 32 >= r.cnt) w.y = 0.0f;
-                part = add2(part, w);
-                if (++np == kGiantFold) {
-                    float err;
-                    s = two_sum(s, part.x + part.y, err);
-                    c += err;
-                    part = f2(0.0f);
-                    np = 0;
-                }
+                const float2 t = add2(ks, w);
+                kc = add2(kc, sub2(w, sub2(t, ks)));
+                ks = t;
             }
-            float err;
-            s = two_sum(s, part.x + part.y, err);
-            c += err;
         }
+        float err;
+        float s = two_sum(ks.x - 1.0f, ks.y - 1.0f, err), c = (kc.x + kc.y) + err;
         warp_sum_ff(s, c);
         const int total = __reduce_add_sync(0xffffffffu, g.cnt);
         if (lane == 0 && total > 0) {
@@ -841,6 +845,7 @@ struct Piece {
     int s, e;    // tile pixels [s, e)
 };
 
+template <int W = kTileW>
 __device__ __forceinline__ Piece piece_of(int p, int lo, int cnt, int nr, int base) {
     // in-ring index of the run's first pixel and the pixels before the wrap
     const int i0 = lo < 0 ? lo + nr : lo;
@@ -849,7 +854,7 @@ __device__ __forceinline__ Piece piece_of(int p, int lo, int cnt, int nr, int ba
     r.a = p ? -base - n0 : i0 - base;
     const int first = p ? -base : r.a, end = p ? cnt - n0 - base : r.a + n0;
     r.s = max(first, 0);
-    r.e = min(end, kTileW);
+    r.e = min(end, W);
     return r;
 }
 
@@ -1130,25 +1135,35 @@ __global__ void __launch_bounds__(kDepWarps * 32, kDepBlocks)
 }
 
 constexpr int kGenWarps = 2;
+constexpr int kPxW = kTileW / 2;
 
-// The general discs on coarser rings, and the giants: the tile in shared memory (one row per lane, rows an odd
-// number of words apart), each pixel's weight from the run-time series, eight
-// pixels at a time.
+// The general discs on coarser rings, and the giants: each pixel's weight from
+// the run-time series, eight pixels at a time, into a pixel in shared memory
+// that is a two-float, added to with TwoSum: one giant can be most of a map's
+// flux, and its FP32 deposits and sums left 1e-9 of it.  A warp takes half of a
+// tile's columns at a time (one row per lane, rows an odd number of words
+// apart): with 8 KB a warp instead of 17 as many are resident as the registers
+// allow.
 __global__ void __launch_bounds__(kGenWarps * 32)
     k_tile_dep_px(const __grid_constant__ DiscArgs a, const __grid_constant__ TileArgs tg) {
     if (tg.ctl[0] != 2) return;
-    constexpr int kRow = kTileW + 1, kStep = 8;
+    constexpr int kRow = kPxW + 1, kStep = 8;
     __shared__ TileHdr sh[kGenWarps][2];
-    __shared__ float tile[kGenWarps][32 * kRow + kStep];
+    __shared__ float2 tile[kGenWarps][32 * kRow];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float *const my = tile[w] + lane * kRow;
-    TileUnit un;
-    while (claim_unit(a, tg, 3, un)) {
-        const int strip = un.tile / tg.ncol, base = (un.tile - strip * tg.ncol) * kTileW;
+    float2 *const my = tile[w] + lane * kRow;
+    const long long halves = 2 * a.ctr[C_UNITS + 3];
+    for (;;) {
+        long long u = 0;
+        if (lane == 0) u = (long long)atomicAdd((unsigned long long *)(a.ctr + C_UNEXT + 3), 1ull);
+        u = __shfl_sync(0xffffffffu, u, 0);
+        if (u >= halves) break;
+        const TileUnit un = tg.units[3 * tg.unit_cap + (u >> 1)];
+        const int strip = un.tile / tg.ncol, base = (un.tile - strip * tg.ncol) * kTileW + (int)(u & 1) * kPxW;
         const int ring = min(strip * kTileR + 1 + lane, a.g.nrings);
         const bool own = strip * kTileR + 1 + lane <= a.g.nrings;
         const RingT rc = ring_t(a, ring);
-        for (int t = 0; t < kTileW; t++) my[t] = 0.0f;
+        for (int t = 0; t < kPxW; t++) my[t] = f2(0.0f);
         for_items(tg, un, sh[w], [&](const TileHdr &h) {
             Run r{};
             int lo = 0, cnt = 0;
@@ -1161,23 +1176,30 @@ __global__ void __launch_bounds__(kGenWarps * 32)
             const float2 F2 = f2(h.F), Fl2 = f2(h.p * (h.Fn - h.F));
 #pragma unroll 1
             for (int p = 0; p < 2; p++) {
-                Piece pc{0, kTileW, 0};
-                if (cnt > 0) pc = piece_of(p, lo, cnt, rc.nr, base);
-                if (pc.e <= pc.s) pc.s = kTileW, pc.e = 0;
+                Piece pc{0, kPxW, 0};
+                if (cnt > 0) pc = piece_of<kPxW>(p, lo, cnt, rc.nr, base);
+                if (pc.e <= pc.s) pc.s = kPxW, pc.e = 0;
                 const int s = __reduce_min_sync(0xffffffffu, pc.s), end = __reduce_max_sync(0xffffffffu, pc.e);
                 for (int t = s; t < end; t += kStep) {
-                    float2 wt[kStep / 2];
+                    float2 wt[kStep / 2], wl[kStep / 2];   // w (F + Flo) as a two-float
 #pragma unroll
                     for (int k = 0; k < kStep / 2; k++) {
                         const float jf = (float)(t + 2 * k - pc.a);
                         const float2 wk = weight2<-1, -1>(e, r, make_float2(jf, jf + 1.0f));
-                        wt[k] = fma2(wk, F2, mul2(wk, Fl2));
+                        wt[k] = mul2(wk, F2);
+                        wl[k] = fma2(wk, Fl2, fma2(wk, F2, make_float2(-wt[k].x, -wt[k].y)));
                     }
+                    auto add = [&](int at, float v, float lo) {
+                        if (at < pc.s || at >= pc.e) return;
+                        const float2 m = my[at];
+                        float err;
+                        const float sum = two_sum(m.x, v, err);
+                        my[at] = make_float2(sum, m.y + (err + lo));
+                    };
 #pragma unroll
                     for (int k = 0; k < kStep / 2; k++) {
-                        const int t0 = t + 2 * k, t1 = t0 + 1;
-                        if (t0 >= pc.s && t0 < pc.e) my[t0] += wt[k].x;
-                        if (t1 >= pc.s && t1 < pc.e) my[t1] += wt[k].y;
+                        add(t + 2 * k, wt[k].x, wl[k].x);
+                        add(t + 2 * k + 1, wt[k].y, wl[k].y);
                     }
                 }
             }
@@ -1186,15 +1208,13 @@ __global__ void __launch_bounds__(kGenWarps * 32)
         __syncwarp();
         for (int r = 0; r < kTileR; r++) {
             const long long p = __shfl_sync(0xffffffffu, row, r);
-#pragma unroll
-            for (int k = 0; k < kTileW / 32; k++) {
-                const float v = tile[w][r * kRow + 32 * k + lane];
-                if (v != 0.0f) red_add_f64(a.acc.acc64 + (p + 32 * k + lane), (double)v);
-            }
+            const float2 v = tile[w][r * kRow + lane];
+            if (v.x != 0.0f) red_add_f64(a.acc.acc64 + (p + lane), (double)v.x + (double)v.y);
         }
         __syncwarp();
     }
 }
+static_assert(kPxW == 32, "a lane per column of the half");
 
 template <class K>
 int resident(K k, int threads) {

@@ -174,7 +174,9 @@ static_assert(sizeof(TileHdr) == 64, "four 16-byte words");
 
 struct TileArgs {
     TileHdr *hdr;             // per block-class disc
-    const int *ctl;           // SegArgs::ctl: 2 when the chunk is rendered by tiles
+    int *ctl;                 // SegArgs::ctl: [0] 2 when the chunk is rendered by tiles, [2] discs that
+                              // are giants by their flux
+    const double *flux_sum;   // flux kept so far
     int nstrips, ncol;        // tiles of the map: strips of kTileR rings x columns
     unsigned *list;           // the pairs' discs, tile by tile
     unsigned *hist;           // [kTileLists][tiles][kTileClasses]: pairs per octave, then list slots

@@ -48,3 +48,15 @@ def test_full_rings(rend, nside, lo, hi):
     z = np.cos(rng.uniform(0.002, 0.9 * lo, n)) * rng.choice([-1.0, 1.0], n)
     radius = np.exp(rng.uniform(math.log(lo), math.log(hi), n))
     assert abs(flux_error(rend, discs(z, rng.uniform(0, 6.28, n), radius, rng), nside)) <= 1e-9
+
+
+# A disc that is the whole map's flux is summed over its pixels and deposited in
+# two-floats: 2^-46 for each of the sums, the quotient and the deposits, which
+# is 1e-13, and FP64 sums of up to 3e6 pixels: 1e-11 leaves ten times that.
+@pytest.mark.parametrize("nside", [64, 512])
+@pytest.mark.parametrize("theta,phi,radius", [
+    (1.4, 3.14159, 0.1), (0.002, 1.0, 0.15), (0.84, 0.0, 0.12), (1.57, 1.0, 0.31), (1.0, 3.14, 0.7),
+    (0.5, 2.0, 1.3), (1.2, 4.0, 2.1), (1.2, 4.0, 2.6), (2.0, 0.5, 3.3)])
+def test_one_disc(rend, nside, theta, phi, radius):
+    parts = discs(np.array([math.cos(theta)]), np.array([phi]), np.array([radius]), np.random.default_rng(1))
+    assert abs(flux_error(rend, parts, nside)) <= 1e-11
