@@ -437,6 +437,7 @@ dmann_status dmann_create(dmann_ctx **out, int device) {
     ctx->tune.blocks_per_sm = 0;
     ctx->tune.ring_chunk = 384;
     ctx->tune.seg_min_deposits_log2 = 28;
+    ctx->tune.large_render = kLargeAny;
     *out = ctx;
     return DMANN_OK;
 }
@@ -552,6 +553,7 @@ dmann_status merge_tuning(dmann_ctx *ctx, const dmann_tuning &t, dmann_tuning &d
     if (t.warp_max_pixels > 0) dst.warp_max_pixels = t.warp_max_pixels;
     if (t.blocks_per_sm > 0) dst.blocks_per_sm = t.blocks_per_sm;
     if (t.block_threads > 0) dst.block_threads = t.block_threads;
+    if (t.large_render >= kLargeAny && t.large_render <= kLargeSegments) dst.large_render = t.large_render;
     dst.ring_chunk = dst.block_threads == 128 ? 192 : dst.block_threads == 512 ? 640 : 384;
     return DMANN_OK;
 }
@@ -790,8 +792,9 @@ bool may_be_large(size_t n, int nside, const dmann_tuning &tu) {
 
 bool reserve_large(dmann_ctx *ctx, size_t n, int nside, const dmann_tuning &tu) {
     if (!may_be_large(n, nside, tu)) return true;
-    const bool tile = have_tile(ctx, n, nside, true);
-    return (tile && tile_always_fits(n, nside)) || have_seg(ctx, n, nside, true) || tile;
+    const bool tile = tu.large_render != kLargeSegments && have_tile(ctx, n, nside, true);
+    const bool seg = tu.large_render != kLargeTiles;
+    return (tile && tile_always_fits(n, nside)) || (seg && have_seg(ctx, n, nside, true)) || tile;
 }
 
 // The compensated form's block-class discs of a chunk that may be large:
@@ -812,8 +815,9 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     const int nside = ctx->g.nside;
     if (!da.chdr || !may_be_large(N, nside, tu)) return DMANN_OK;
     Work &w = *ctx->w;
-    const bool have_t = have_tile(ctx, N, nside, grow), fits = tile_always_fits(N, nside);
-    const auto [tile, seg, count] = plan_large(have_t, fits, !(have_t && fits) && have_seg(ctx, N, nside, grow));
+    const bool have_t = tu.large_render != kLargeSegments && have_tile(ctx, N, nside, grow);
+    const bool fits = tile_always_fits(N, nside), want_s = tu.large_render != kLargeTiles && !(have_t && fits);
+    const auto [tile, seg, count] = plan_large(have_t, fits, want_s && have_seg(ctx, N, nside, grow));
     if (!tile && !seg) return DMANN_OK;
     cudaStream_t s = ctx->stream;
     const int bt = tu.block_threads == 128 ? 128 : 256;

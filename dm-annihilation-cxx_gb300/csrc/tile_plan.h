@@ -37,6 +37,9 @@ inline size_t tile_unit_capacity(size_t n, int nside) {
 }
 inline bool tile_always_fits(size_t n, int nside) { return tile_capacity(n, nside) == tile_pairs_bound(n, nside); }
 
+// dmann_tuning.large_render
+enum { kLargeAny = 1, kLargeTiles = 2, kLargeSegments = 3 };
+
 // The renders launched for a chunk that may be large, from the buffers there
 // are: the segments are of use where the pair list can overflow, and there the
 // chunk's pairs are counted whether or not there are segments to take it -- the

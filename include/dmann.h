@@ -115,7 +115,7 @@ typedef struct {
 
 /* Tunables (set by the annmap autotuner; zero fields keep the current
  * values).  Defaults: warp_max_pixels 1024, block_threads 256, blocks_per_sm
- * 0 (as many as fit), seg_min_deposits_log2 28. */
+ * 0 (as many as fit), seg_min_deposits_log2 28, large_render 1. */
 typedef struct {
     int64_t warp_max_pixels;   /* footprint-class bin edge: discs estimated up
                                   to this many pixels go warp-per-particle,
@@ -133,7 +133,13 @@ typedef struct {
                                   lists would not fit): short FP32 sums added
                                   into the FP64 plane; smaller chunks deposit
                                   in FP64.  1 .. 62 */
-    int32_t reserved[2];
+    int32_t large_render;      /* compensated form: the render of the chunks that
+                                  reach seg_min_deposits_log2.  1 (default):
+                                  tiles where they fit, else segments; 2: never
+                                  segments; 3: never tiles; other values keep
+                                  the current one.  A chunk that its render
+                                  cannot hold deposits in FP64 */
+    int32_t reserved;
 } dmann_tuning;
 
 /* ---- lifetime ---- */
