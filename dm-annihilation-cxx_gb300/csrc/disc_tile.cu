@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(256) k_tile_hdr(DiscArgs a, TileArgs tg) {
         t.hR = c.ch.hR;
         t.sth0 = c.ch.sth0;
         t.nK = c.ext.nK;
-        t.F = t.Fn = t.p = 0.0f;
+        t.F = t.Flo = t.sh = 0.0f;
         const double turns = c.hdr.phi0 * kInvTwoPi;
         t.ph = (float)turns;
         t.pl = (float)(turns - (double)t.ph);
@@ -644,34 +644,60 @@ __global__ void __launch_bounds__(kNormWarps * 32)
 // F = flux / S into the disc's tile header; a disc of fewer than two pixels
 // puts its whole flux into the centre pixel (genmap.cpp:125-128) and has
 // F = 0.  Also the chunk's largest octave of F.
+//
+// A deposit is one FMA with a float, and F rounded to one would be an error of
+// up to 2^-24 in each of a disc's pixels (a two-float F took two more packed
+// operations per pixel pair and 9 % more time).  w F = 2^(t + s) (2^-s F), so
+// of kShifts small shifts s of the disc's exponents, which cost nothing, the one
+// is taken whose 2^-s F is nearest to a float: within 2^-24 / kShifts on
+// average.  The shifts are of either sign, so that ex2's errors on either side
+// of an octave stay as the weight sums have them.
+constexpr int kShifts = 16;
+__device__ __forceinline__ float shift_of(int k) { return (float)(k - kShifts / 2) * (1.0f / 256.0f); }
+
 __global__ void __launch_bounds__(256) k_tile_fin(DiscArgs a, TileArgs tg) {
     if (tg.ctl[0] != 2) return;
     const long long nblk = a.ctr[C_ADD_BLOCK];
     const long long stride = (long long)gridDim.x * blockDim.x;
+    __shared__ float2 pow2[kShifts];   // 2^-shift as a two-float
+    if (threadIdx.x < kShifts) {
+        const double v = exp2(-(double)shift_of(threadIdx.x));
+        pow2[threadIdx.x].x = (float)v;
+        pow2[threadIdx.x].y = (float)(v - (double)(float)v);
+    }
+    __syncthreads();
     int oct = 0;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nblk; q += stride) {
         const DiscHdr &d = a.chdr[q].hdr;
         const double fs = d.flux * a.f.inv_scale;
         const long long px = tg.disc_px[q];
-        float F = 0.0f, Fn = 0.0f, p = 0.0f;
+        float F = 0.0f, Flo = 0.0f, sh = 0.0f;
+        TileHdr &t = tg.hdr[q];
         if (px < 2) {
             red_add_f64(a.acc.acc64 + d.cpix, fs);
             atomicAdd((unsigned long long *)(a.ctr + C_DEPOSITS), (unsigned long long)(1 - px));
         } else {
-            // F between the neighbouring floats F and Fn, p of the way
             const double Fd = fs / tg.disc_S[q];
             F = (float)Fd;
-            const double r = Fd - (double)F;
-            if (F != 0.0f && isfinite(F)) {
-                Fn = __int_as_float(__float_as_int(F) + ((r > 0.0) == (F > 0.0f) ? 1 : -1));
-                p = (float)(r / ((double)Fn - (double)F));
-                if (!isfinite(Fn)) p = 0.0f;
+            Flo = (float)(Fd - (double)F);
+            if ((t.flags & kKindMask) != K_GIANT && Flo != 0.0f) {
+                const float Fh = F, Fl = Flo;
+                float best = fabsf(Flo);
+                for (int k = 0; k < kShifts; k++) {
+                    const float2 g = pow2[k];
+                    const float v = Fh * g.x, e = fmaf(Fh, g.x, -v) + fmaf(Fh, g.y, Fl * g.x);
+                    if (fabsf(e) < best) {
+                        best = fabsf(e);
+                        F = v;
+                        Flo = e;
+                        sh = shift_of(k);
+                    }
+                }
             }
         }
-        TileHdr &t = tg.hdr[q];
         t.F = F;
-        t.Fn = Fn;
-        t.p = p;
+        t.Flo = Flo;
+        t.sh = sh;
         oct = max(oct, (int)((__float_as_uint(F) >> 23) & 255));
     }
     oct = __reduce_max_sync(0xffffffffu, oct);
@@ -946,7 +972,7 @@ __device__ __noinline__ float2 gen_exponent(float nK, int tier_x, int tier_h, fl
 }
 
 __device__ __forceinline__ void add_gen(float2 (&acc)[kTileW / 2], const Piece &pc, const Ext &e, const Run &r,
-                                        float2 F) {
+                                        float2 F, float shift) {
     // near Chebyshev points (0.966, 0.707, 0.259 of 16 pixels) exact in FP32,
     // squares too; the reciprocals as FP32 pairs: an error of these constants
     // would be the same in every disc
@@ -979,7 +1005,8 @@ __device__ __forceinline__ void add_gen(float2 (&acc)[kTileW / 2], const Piece &
         const float2 d23 = fma2(s23, f2(i23), mul2(s23, f2(i23l)));
         const float2 q2 = mul2(sub2(fma2(s12, f2(i12), mul2(s12, f2(i12l))), d23), f2(i13));
         const float2 q1 = fma2(q2, f2(-(m2 + m3)), d23);
-        const float2 q0 = fma2(f2(-m3), fma2(q2, f2(-m2), d23), p3);
+        float2 q0 = fma2(f2(-m3), fma2(q2, f2(-m2), d23), p3);
+        q0.x += shift;
 #pragma unroll
         for (int gg = 0; gg < kSubPx / kGroupPx; gg++) {
             const int gi = b * (kSubPx / kGroupPx) + gg;
@@ -1031,19 +1058,6 @@ __device__ __forceinline__ void for_items(const TileArgs &tg, const TileUnit &un
     }
 }
 
-// F lies between two floats: a share p of the deposits takes the further
-// one, by the golden ratio's sequence over the rings (half a turn apart for
-// even and odd pixels of the tile), so that a disc's deposits add up to its
-// flux although each is one FMA with one float (a two-float F took two more
-// packed operations per pixel pair and 9 % more time).
-__device__ __forceinline__ float2 ring_phase(int ring) {
-    const float v = (float)ring * 0.61803399f, a = v - floorf(v);
-    return make_float2(a, a < 0.5f ? a + 0.5f : a - 0.5f);
-}
-__device__ __forceinline__ float2 disc_F(const TileHdr &h, float2 phase) {
-    return make_float2(h.p > phase.x ? h.Fn : h.F, h.p > phase.y ? h.Fn : h.F);
-}
-
 // Units of one list: 0 and 1 polynomial discs (K_POLY3, K_POLY), 2 general
 // discs on fine rings, 3 the other general discs and the giants.  (Each list
 // has a kernel of its own: together they do not fit the instruction cache.)
@@ -1074,7 +1088,6 @@ __global__ void __launch_bounds__(kDepWarps * 32, kDepBlocks)
         const int ring = min(strip * kTileR + 1 + lane, a.g.nrings);
         const bool own = strip * kTileR + 1 + lane <= a.g.nrings;
         const RingT rc = ring_t(a, ring);
-        const float2 phase = ring_phase(ring);
         float2 acc[kTileW / 2];
 #pragma unroll
         for (int k = 0; k < kTileW / 2; k++) acc[k] = f2(0.0f);
@@ -1085,7 +1098,7 @@ __global__ void __launch_bounds__(kDepWarps * 32, kDepBlocks)
             if (own && ring >= h.r_first && ring <= h.r_last)
                 cnt = max(0, tile_run<GEN>(a, h, rc, ring, lo, r.d0h, r.A, r.B));
             __syncwarp();
-            const float2 F = disc_F(h, phase);
+            const float2 F = f2(h.F);
             Piece pc{0, 0, 0};
             if (cnt > 0) pc = piece_of(0, lo, cnt, rc.nr, base);
             const bool second = __any_sync(0xffffffffu, cnt > 0 && (lo < 0 || lo + cnt > rc.nr));
@@ -1098,11 +1111,12 @@ __global__ void __launch_bounds__(kDepWarps * 32, kDepBlocks)
                 e = gen_ext(a, h);
             } else {
                 poly_coeffs(r.A, r.B, h.nK, LIST == 1 && (h.flags & kFlagH1) ? 1 : 0, co);
+                co[0] += h.sh;
             }
 #pragma unroll 1
             for (int p = 0;; p++) {
                 if (some) {
-                    if constexpr (GEN) add_gen(acc, pc, e, r, F);
+                    if constexpr (GEN) add_gen(acc, pc, e, r, F, h.sh);
                     else add_poly<LIST == 0>(acc, pc, co, r.d0h, r.steph, F);
                 }
                 if (p == 1 || !second) break;
@@ -1173,7 +1187,7 @@ __global__ void __launch_bounds__(kGenWarps * 32)
             r.steph = 0.5f * rc.step;
             if (h.flags & kFlagA2) r.A2 = antipode_term(h, rc);
             const Ext e = gen_ext(a, h);
-            const float2 F2 = f2(h.F), Fl2 = f2(h.p * (h.Fn - h.F));
+            const float2 F2 = f2(h.F), Fl2 = f2(h.Flo), sh2 = f2(h.sh);
 #pragma unroll 1
             for (int p = 0; p < 2; p++) {
                 Piece pc{0, kPxW, 0};
@@ -1185,7 +1199,8 @@ __global__ void __launch_bounds__(kGenWarps * 32)
 #pragma unroll
                     for (int k = 0; k < kStep / 2; k++) {
                         const float jf = (float)(t + 2 * k - pc.a);
-                        const float2 wk = weight2<-1, -1>(e, r, make_float2(jf, jf + 1.0f));
+                        float2 sn, hv, g;
+                        const float2 wk = ex2_2(add2(exponent2x<-1, -1>(e, r, make_float2(jf, jf + 1.0f), sn, hv, g), sh2));
                         wt[k] = mul2(wk, F2);
                         wl[k] = fma2(wk, Fl2, fma2(wk, F2, make_float2(-wt[k].x, -wt[k].y)));
                     }

@@ -165,7 +165,7 @@ struct alignas(16) TileHdr {
     float t0h, t0l;         // theta0 as a two-float
     float hR, sth0;         // hav(R), sin(theta0)
     float nK;
-    float F, Fn, p;         // flux / S lies a share p of the way from F to its neighbour Fn
+    float F, Flo, sh;       // flux / S = 2^sh (F + Flo)
     float ph, pl;           // phi0 / 2 pi as a two-float
     int r_first, r_last, irmin, irmax;   // as DiscHdr
     int q, flags;           // queue slot; kind and flags (disc_tile.cu)
