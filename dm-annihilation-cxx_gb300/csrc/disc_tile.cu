@@ -62,7 +62,7 @@ enum Kind {
     K_GIANT = 3    // the same, summed pixel by pixel and deposited in two floats: radius beyond
                    // kGiantR (which may reach the kink at the antipode), or a share of the map's flux
 };
-constexpr int kKindMask = 3, kFlagH1 = 4, kFlagAll = 8, kFlagFast = 16, kFlagA2 = 32;
+constexpr int kKindMask = 3, kFlagH1 = 4, kFlagAll = 8, kFlagFast = 16, kFlagA2 = 32, kFlagLong = 64;
 constexpr double kGiantR = 2.2;
 
 // Discs with 1 / kShare and more of the flux kept so far are giants too.  The
@@ -80,6 +80,8 @@ constexpr int kShare = 256, kShareMax = 1024;
 // against the FP64 form is the same (Nside 512: 4.8e-8 with, 5.5e-8 without;
 // 2048: 8.1e-8 and 8.0e-8, 1.06e-7 and 1.06e-7).
 constexpr float kPoly3Sin = 0.1987f;
+
+constexpr int kLongRings = 256;   // general discs of more are summed by several warps
 
 // Rings from which a general disc's exponent is interpolated over 32 pixels
 // (half azimuth offsets of 16 pixels below 0.06 rad: see add_gen).
@@ -464,6 +466,10 @@ __global__ void __launch_bounds__(256) k_tile_hdr(DiscArgs a, TileArgs tg) {
             kind = K_GIANT;
         t.flags = kind | (c.ext.tier_h >= 1 ? kFlagH1 : 0) | (c.hdr.allsky ? kFlagAll : 0) |
                   (c.ch.fast ? kFlagFast : 0) | (c.ext.tier_h == 2 ? kFlagA2 : 0);
+        if (kind == K_GEN && t.r_last - t.r_first >= kLongRings) {
+            t.flags |= kFlagLong;
+            tg.gen[nblk - 1 - atomicAdd(tg.ctl + 3, 1)] = (int)q;
+        }
         tg.hdr[q] = t;
         if (kind == K_GIANT) {
             const unsigned long long k = atomicAdd((unsigned long long *)(a.ctr + C_GEN), 1ull);
@@ -491,11 +497,14 @@ __device__ __forceinline__ Ext gen_ext(const DiscArgs &a, const TileHdr &h) { re
 
 constexpr int kNormWarps = 4;
 constexpr int kNormClaim = 4;   // discs per claim
+constexpr int kLongParts = 32;  // claims per general disc of more than kLongRings rings
 
 // S and the pixel count of every disc but the giants: a warp per disc, a ring
 // per lane.  5.6 ms, bound by FP32 issue (the ring's chord test and 8 or 12
 // node values; the segmented render's first pass visits every pixel: 0.41 s
-// on the whole set).
+// on the whole set).  A general disc of R = 2 at Nside 1522 has 3900 rings, 26 us
+// for each 32 of them: on one warp it took 2.9 ms, half of a map of 3000
+// particles.  The long ones come first, in parts.
 __global__ void __launch_bounds__(kNormWarps * 32, 7)
     k_tile_norm(const __grid_constant__ DiscArgs a, const __grid_constant__ TileArgs tg) {
     if (tg.ctl[0] != 2) return;
@@ -503,71 +512,99 @@ __global__ void __launch_bounds__(kNormWarps * 32, 7)
     const int lane = threadIdx.x & 31;
     TileHdr &h = sh[threadIdx.x >> 5];
     const Dither mine = lane_dither();
-    const long long nblk = a.ctr[C_ADD_BLOCK];
-    long long deposits = 0;
+    const long long nblk = a.ctr[C_ADD_BLOCK], nparts = (long long)tg.ctl[3] * kLongParts;
+    auto claim = [&](unsigned long long *next, int k) {
+        long long t = 0;
+        if (lane == 0) t = (long long)atomicAdd(next, (unsigned long long)k);
+        return __shfl_sync(0xffffffffu, t, 0);
+    };
+    long long deposits = 0, next = 0, end = 0;
+    bool parts = nparts > 0;
     for (;;) {
-        long long q0 = 0;
-        if (lane == 0) q0 = (long long)atomicAdd((unsigned long long *)(a.ctr + C_TILE_NEXT), (unsigned long long)kNormClaim);
-        q0 = __shfl_sync(0xffffffffu, q0, 0);
-        if (q0 >= nblk) break;
-        const long long q1 = min(nblk, q0 + kNormClaim);
-        for (long long q = q0; q < q1; q++) {
-            __syncwarp();
-            load_thdr(tg, q, h);
-            __syncwarp();
-            const int kind = h.flags & kKindMask;
-            if (kind == K_GIANT) continue;
-            const Dither di = deal_dither(mine, q);
-            float s = 0.0f, c = 0.0f;
-            int total = 0;
-            const int r_last = h.r_last;
-            if (kind <= K_POLY) {
-                const int th = (h.flags & kFlagH1) ? 1 : 0;
-                const float nK = h.nK;
-                for (int r0 = h.r_first; r0 <= r_last; r0 += 32) {
-                    const int ring = r0 + lane;
-                    if (ring > r_last) continue;
-                    const RingT rc = ring_t(a, ring);
-                    int lo;
-                    float d0h, A, B;
-                    const int cnt = tile_run<false>(a, h, rc, ring, lo, d0h, A, B);
-                    if (cnt <= 0) continue;
-                    float co[5];
-                    poly_coeffs(A, B, nK, th, co);
-                    if (kind == K_POLY3) co[4] = 0.0f;   // (the deposits' polynomial)
-                    const float2 v = ring_sum(co, d0h, 0.5f * rc.step, cnt, di);
-                    total += cnt;
-                    float err;
-                    s = two_sum(s, v.x, err);
-                    c += err + v.y;
-                }
-            } else {
-                const Ext e = gen_ext(a, h);
-                for (int r0 = h.r_first; r0 <= r_last; r0 += 32) {
-                    const int ring = r0 + lane;
-                    if (ring > r_last) continue;
-                    const RingT rc = ring_t(a, ring);
-                    Run g{};
-                    int lo;
-                    g.cnt = tile_run<true>(a, h, rc, ring, lo, g.d0h, g.A, g.B);
-                    if (g.cnt <= 0) continue;
-                    g.steph = 0.5f * rc.step;
-                    if (h.flags & kFlagA2) g.A2 = antipode_term(h, rc);
-                    const float2 v = ring_sum_gen(e, g, ring < h.irmin || ring > h.irmax, di);
-                    total += g.cnt;
-                    float err;
-                    s = two_sum(s, v.x, err);
-                    c += err + v.y;
-                }
+        long long q;
+        int part = -1;
+        if (parts) {
+            const long long t = claim((unsigned long long *)(tg.ctl + 4), 1);
+            if (t >= nparts) {
+                parts = false;
+                continue;
             }
-            __syncwarp();
-            warp_sum_ff(s, c);
-            total = __reduce_add_sync(0xffffffffu, total);
-            if (lane == 0) {
+            q = tg.gen[nblk - 1 - t / kLongParts];
+            part = (int)(t % kLongParts);
+        } else {
+            if (next == end) {
+                next = claim((unsigned long long *)(a.ctr + C_TILE_NEXT), kNormClaim);
+                if (next >= nblk) break;
+                end = min(nblk, next + kNormClaim);
+            }
+            q = next++;
+        }
+        __syncwarp();
+        load_thdr(tg, q, h);
+        __syncwarp();
+        const int kind = h.flags & kKindMask;
+        if (kind == K_GIANT || (part < 0 && (h.flags & kFlagLong))) continue;
+        int r_first = h.r_first, r_last = h.r_last;
+        if (part >= 0) {   // whole warps of rings per part
+            const int step = ((r_last - r_first) / (32 * kLongParts) + 1) * 32;
+            r_first += part * step;
+            r_last = min(r_last, r_first + step - 1);
+            if (r_first > r_last) continue;
+        }
+        const Dither di = deal_dither(mine, q);
+        float s = 0.0f, c = 0.0f;
+        int total = 0;
+        if (kind <= K_POLY) {
+            const int th = (h.flags & kFlagH1) ? 1 : 0;
+            const float nK = h.nK;
+            for (int r0 = r_first; r0 <= r_last; r0 += 32) {
+                const int ring = r0 + lane;
+                if (ring > r_last) continue;
+                const RingT rc = ring_t(a, ring);
+                int lo;
+                float d0h, A, B;
+                const int cnt = tile_run<false>(a, h, rc, ring, lo, d0h, A, B);
+                if (cnt <= 0) continue;
+                float co[5];
+                poly_coeffs(A, B, nK, th, co);
+                if (kind == K_POLY3) co[4] = 0.0f;   // (the deposits' polynomial)
+                const float2 v = ring_sum(co, d0h, 0.5f * rc.step, cnt, di);
+                total += cnt;
+                float err;
+                s = two_sum(s, v.x, err);
+                c += err + v.y;
+            }
+        } else {
+            const Ext e = gen_ext(a, h);
+            for (int r0 = r_first; r0 <= r_last; r0 += 32) {
+                const int ring = r0 + lane;
+                if (ring > r_last) continue;
+                const RingT rc = ring_t(a, ring);
+                Run g{};
+                int lo;
+                g.cnt = tile_run<true>(a, h, rc, ring, lo, g.d0h, g.A, g.B);
+                if (g.cnt <= 0) continue;
+                g.steph = 0.5f * rc.step;
+                if (h.flags & kFlagA2) g.A2 = antipode_term(h, rc);
+                const float2 v = ring_sum_gen(e, g, ring < h.irmin || ring > h.irmax, di);
+                total += g.cnt;
+                float err;
+                s = two_sum(s, v.x, err);
+                c += err + v.y;
+            }
+        }
+        __syncwarp();
+        warp_sum_ff(s, c);
+        total = __reduce_add_sync(0xffffffffu, total);
+        if (lane == 0) {
+            if (part < 0) {
                 tg.disc_S[q] = (double)s + (double)c;
                 tg.disc_px[q] = total;
-                deposits += total;
+            } else {
+                atomicAdd(tg.disc_S + q, (double)s + (double)c);
+                atomicAdd((unsigned long long *)(tg.disc_px + q), (unsigned long long)total);
             }
+            deposits += total;
         }
     }
     if (lane == 0 && deposits) atomicAdd((unsigned long long *)(a.ctr + C_DEPOSITS), (unsigned long long)deposits);

@@ -31,7 +31,7 @@ constexpr size_t kSegClsBytes = 2 * 4 * kClasses;
 constexpr size_t kSegClsPxBytes = 8 * kClasses;
 constexpr size_t kSegNextBytes = 8 * kSegSlots;
 constexpr size_t kSegSpanBytes = 24 * kSegSlots;
-constexpr size_t kSegBufBytes = kSegClsBytes + kSegClsPxBytes + kSegNextBytes + kSegSpanBytes + 16;
+constexpr size_t kSegBufBytes = kSegClsBytes + kSegClsPxBytes + kSegNextBytes + kSegSpanBytes + 32;
 
 // Device counters (int64).  The first six accumulate over every chunk of
 // a map; the ones from C_ADD_DISC on describe the chunk being added and are
@@ -175,7 +175,7 @@ static_assert(sizeof(TileHdr) == 64, "four 16-byte words");
 struct TileArgs {
     TileHdr *hdr;             // per block-class disc
     int *ctl;                 // SegArgs::ctl: [0] 2 when the chunk is rendered by tiles, [2] discs that
-                              // are giants by their flux
+                              // are giants by their flux, [3] long general discs, [4, 5] their parts claimed
     const double *flux_sum;   // flux kept so far
     int nstrips, ncol;        // tiles of the map: strips of kTileR rings x columns
     unsigned *list;           // the pairs' discs, tile by tile
@@ -185,7 +185,8 @@ struct TileArgs {
     long long unit_cap;
     double *disc_S;           // per block-class disc, as SegArgs
     long long *disc_px;
-    int *gen;                 // queue slots of the giant discs (C_GEN of them)
+    int *gen;                 // queue slots of the giant discs (C_GEN, from the front) and of the long
+                              // general discs (from the end of the block class)
 };
 
 // prep.cu

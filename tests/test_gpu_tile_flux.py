@@ -60,3 +60,26 @@ def test_full_rings(rend, nside, lo, hi):
 def test_one_disc(rend, nside, theta, phi, radius):
     parts = discs(np.array([math.cos(theta)]), np.array([phi]), np.array([radius]), np.random.default_rng(1))
     assert abs(flux_error(rend, parts, nside)) <= 1e-11
+
+
+# The discs of test_gpu_tiles.py's test_single_disc 400 times over, so that none
+# has 1/256 of the flux and they take the polynomial and general paths, the
+# longer general ones (beyond 256 rings) summed in parts: against one disc of the
+# plain form, the same pixels, deposits and bounds.
+@pytest.mark.parametrize("nside", [64, 512])
+@pytest.mark.parametrize("theta,phi,radius", [
+    (1.4, 3.14159, 0.1), (1.4, 3.1, 0.24), (0.002, 1.0, 0.15), (0.2, 3.14, 0.15), (3.0, 2.0, 0.3),
+    (0.84, 0.0, 0.12), (2.3, 3.2, 0.27), (1.57, 1.0, 0.31), (1.0, 3.14, 0.7), (0.5, 2.0, 1.3),
+    (1.2, 4.0, 2.1), (1.2, 4.0, 2.6), (2.0, 0.5, 3.3)])
+def test_copies_of_a_disc(rend, nside, theta, phi, radius):
+    n = 400
+    one = discs(np.array([math.cos(theta)]), np.array([phi]), np.array([radius]), np.random.default_rng(1))
+    parts = {k: np.repeat(v, n) for k, v in one.items()}
+    assert abs(flux_error(rend, parts, nside)) <= 6e-8
+    got = rend.render(parts, nside, COMP)
+    st = rend.stats()
+    ref = n * rend.render(one, nside, annmap.PLAIN_F64)
+    assert st["deposits"] == n * rend.stats()["deposits"]
+    assert np.array_equal(got != 0, ref != 0)
+    at = ref > 0
+    assert (np.abs(got[at] - ref[at]) / ref[at]).max() <= 1e-5
