@@ -403,8 +403,9 @@ __device__ void adjc_particle(const adj::AdjArgs &a, AdjcSmem<RCH> &sm, long lon
 }
 
 // The gradients of the disc particles from their sums (FP64), one thread per
-// disc, and the observer terms.
-__global__ void __launch_bounds__(128) k_adjc_grad(adj::AdjArgs a, const AdjSums *sums) {
+// disc, and the observer terms.  Blocks of one warp for small sets, as k_comp_hdr.
+template <int BT>
+__global__ void __launch_bounds__(BT) k_adjc_grad(adj::AdjArgs a, const AdjSums *sums) {
     __shared__ double red[12][32];
     double acc[12] = {0.0};
     const long long ndisc = a.d.ctr[C_ADD_DISC];
@@ -436,13 +437,18 @@ __global__ void __launch_bounds__(128) k_adjc_grad(adj::AdjArgs a, const AdjSums
         const double KV[3] = {K * V[0], K * V[1], K * V[2]};
         adj::write_grad(a, i, Gm * a.inv_dOmega, K * s.t, KV, true, acc);
     }
-    adj::group_sum<128, 12>(acc, red);
+    adj::group_sum<BT, 12>(acc, red);
     if (threadIdx.x == 0) adj::flush_acc(a.oacc, acc);
 }
 
-// One block per disc of the block class.  1M particles at Nside 512 (1024
-// threads a SM, 64 registers each): 45.7 ms with blocks of 128 threads, 49.1
-// with 256, whose barriers wait for more warps, and 47.3 with 64.
+// One block per disc of the block class (1024 threads a SM, 64 registers each).
+// 1M particles at Nside 512: 45.7 ms with blocks of 128 threads, 49.1 with 256,
+// whose barriers wait for more warps, and 47.3 with 64.  Smaller sets wait for
+// their largest discs, which wider blocks finish sooner: at Nside 486 4,189
+// particles take 0.91 ms with 128 threads and 0.60 with 256, 200,001 take 12.9
+// and 8.8 ms.
+constexpr int kAdjWideMax = 1 << 18;   // particles up to which the blocks are of 256 threads
+
 template <int BT, int RCH, int MINB>
 __global__ void __launch_bounds__(BT, MINB) k_adjc_block(adj::AdjArgs a, AdjSums *sums) {
     __shared__ AdjcSmem<RCH> sm;
@@ -548,19 +554,23 @@ cudaError_t launch_adjoint_comp_discs(const adj::AdjArgs &a, void *sum_buf, int 
     AdjSums *const sums = (AdjSums *)sum_buf;
     cudaError_t e = launch_hdr(a.d, num_sms, s);
     if (e != cudaSuccess) return e;
-    int occ = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adjc_block<128, 128, 8>, 128, 0);
+    auto blocks = [&](auto kernel, int threads) {
+        int occ = 0;
+        const cudaError_t r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, 0);
+        if (r != cudaSuccess) return r;
+        kernel<<<num_sms * (occ < 1 ? 1 : occ), threads, 0, s>>>(a, sums);
+        return cudaGetLastError();
+    };
+    e = a.p.n <= kAdjWideMax ? blocks(k_adjc_block<256, 256, 4>, 256) : blocks(k_adjc_block<128, 128, 8>, 128);
     if (e != cudaSuccess) return e;
-    if (occ < 1) occ = 1;
-    k_adjc_block<128, 128, 8><<<num_sms * occ, 128, 0, s>>>(a, sums);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int occw = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occw, k_adjc_warp, kWPBA * 32, 0);
     if (e != cudaSuccess) return e;
     if (occw < 1) occw = 1;
     k_adjc_warp<<<num_sms * occw, kWPBA * 32, 0, s>>>(a, sums);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_adjc_grad<<<num_sms * 8, 128, 0, s>>>(a, sums);
+    if (a.p.n <= num_sms * 256) k_adjc_grad<32><<<num_sms * 8, 32, 0, s>>>(a, sums);
+    else k_adjc_grad<128><<<num_sms * 8, 128, 0, s>>>(a, sums);
     return cudaGetLastError();
 }
 
