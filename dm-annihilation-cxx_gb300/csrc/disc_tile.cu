@@ -41,9 +41,9 @@
 // workload holds 130 pixels on average: 8 packed evaluations in its place.
 //
 // FP32 sums of a tile.  A unit's discs are visited in ascending octave of F
-// and at most kUnitMax of them go into one FP32 sum: an addend (w >= exp(-6))
-// is never below 2^-20 of its pixel's total, so no small deposit is lost on a
-// large total, and the rounding errors of the short sums are random.
+// (tile_class in tile_plan.h) and at most kUnitMax of them go into one FP32 sum:
+// no small deposit is lost on a large total, and the rounding errors of the
+// short sums are random.
 #include "comp_engine.cuh"
 
 namespace dmann {
@@ -51,7 +51,7 @@ namespace dmann {
 namespace {
 
 constexpr int kClsBits = 6;
-constexpr int kCls = 1 << kClsBits;   // octaves of F below the chunk's largest
+constexpr int kCls = 1 << kClsBits;   // classes of F (tile_class)
 static_assert(kCls == kTileClasses, "histogram size");
 
 // How a disc's weights are evaluated.
@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(kNormWarps * 32)
 
 // F = flux / S into the disc's tile header; a disc of fewer than two pixels
 // puts its whole flux into the centre pixel (genmap.cpp:125-128) and has
-// F = 0.  Also the chunk's largest octave of F.
+// F = 0.  Also the chunk's largest and smallest octave of F.
 //
 // A deposit is one FMA with a float, and F rounded to one would be an error of
 // up to 2^-24 in each of a disc's pixels (a two-float F took two more packed
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(256) k_tile_fin(DiscArgs a, TileArgs tg) {
         pow2[threadIdx.x].y = (float)(v - (double)(float)v);
     }
     __syncthreads();
-    int oct = 0;
+    int hi = 0, lo = 0;   // largest octave, 255 - the smallest
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nblk; q += stride) {
         const DiscHdr &d = a.chdr[q].hdr;
         const double fs = d.flux * a.f.inv_scale;
@@ -735,10 +735,19 @@ __global__ void __launch_bounds__(256) k_tile_fin(DiscArgs a, TileArgs tg) {
         t.F = F;
         t.Flo = Flo;
         t.sh = sh;
-        oct = max(oct, (int)((__float_as_uint(F) >> 23) & 255));
+        if (F != 0.0f) {
+            const int oct = (int)((__float_as_uint(F) >> 23) & 255);
+            hi = max(hi, oct);
+            lo = max(lo, 255 - oct);
+        }
     }
-    oct = __reduce_max_sync(0xffffffffu, oct);
-    if ((threadIdx.x & 31) == 0 && oct > 0) atomicMax(a.ctr + C_OCT_MAX, (long long)oct);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    lo = __reduce_max_sync(0xffffffffu, lo);
+    if ((threadIdx.x & 31) == 0) {
+        int *const c = reinterpret_cast<int *>(a.ctr + C_OCT);
+        if (hi > 0) atomicMax(c, hi);
+        if (lo > 0) atomicMax(c + 1, lo);
+    }
 }
 
 // ------------------------------------------------------------ pairs
@@ -803,7 +812,8 @@ __global__ void __launch_bounds__(256) k_tile_pairs(DiscArgs a, TileArgs tg) {
     const long long nblk = a.ctr[C_ADD_BLOCK];
     const int sl = threadIdx.x % kPairLanes;
     const long long stride = (long long)gridDim.x * blockDim.x / kPairLanes;
-    const int omax = MODE ? (int)a.ctr[C_OCT_MAX] : 0;
+    const int *const oc = reinterpret_cast<const int *>(a.ctr + C_OCT);
+    const int omax = MODE ? oc[0] : 0, omin = MODE ? 255 - oc[1] : 0;
     const int NT = tg.nstrips * tg.ncol;
     long long total = 0, list[kTileLists] = {};
     for (long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kPairLanes; q < nblk; q += stride) {
@@ -812,7 +822,7 @@ __global__ void __launch_bounds__(256) k_tile_pairs(DiscArgs a, TileArgs tg) {
         if (MODE) {
             const float F = h.F;
             if (F == 0.0f) continue;   // nothing to deposit (weights are >= exp(-6))
-            cls = max(0, kCls - 1 - (omax - (int)((__float_as_uint(F) >> 23) & 255)));
+            cls = tile_class((int)((__float_as_uint(F) >> 23) & 255), omax, omin);
         }
         const int kind = h.flags & kKindMask;
         const int s1 = h.r_last >= h.r_first ? (h.r_last - 1) / kTileR : -1;

@@ -51,7 +51,7 @@ enum Ctr {
     C_TILE_CURSOR,     // pair list slots handed out
     C_UNITS, C_UNEXT = C_UNITS + 4,     // work units of each list, and claims
     C_UNEXT_LAST = C_UNEXT + 3,
-    C_OCT_MAX,         // largest biased FP32 exponent of F
+    C_OCT,             // two ints: the largest biased FP32 exponent of F, 255 - the smallest
     C_COUNT
 };
 constexpr int kCtrChunkFirst = C_ADD_DISC;

@@ -20,6 +20,17 @@ constexpr int kTileLists = 4;
 inline int tile_strips(int nside) { return (4 * nside - 1 + kTileR - 1) / kTileR; }
 inline int tile_cols(int nside) { return (4 * nside + kTileW - 1) / kTileW; }
 
+// The class of a disc in its tile's list, whose classes are summed in ascending
+// order: the biased FP32 exponent oct of its deposit scale below the chunk's
+// largest, omax, in as few octaves per class as hold the smallest, omin (one
+// up to a range of 2^64, four for every float).  So in one FP32 sum of at most
+// kUnitMax discs an addend (weights are above exp(-6) = 2^-8.7) is never below
+// 2^-(9 + 4 + 8.7) of the pixel's total before it, and no small deposit is lost
+// on a large total.
+DMANN_HD inline int tile_class(int oct, int omax, int omin) {
+    return kTileClasses - 1 - (omax - oct) / ((omax - omin) / kTileClasses + 1);
+}
+
 // Every disc of a chunk in every tile.
 inline size_t tile_pairs_bound(size_t n, int nside) {
     return (n > 0 ? n : 1) * (size_t)tile_strips(nside) * (size_t)tile_cols(nside);

@@ -17,4 +17,6 @@ int mode(long long est, long long min_est, long long blocks, long long pairs, lo
          long long item_cap) {
     return large_mode(est, min_est, blocks, pairs, pair_cap, items, item_cap);
 }
+int cls(int oct, int omax, int omin) { return tile_class(oct, omax, omin); }
+int unit_max() { return kUnitMax; }
 }

@@ -1,9 +1,12 @@
 """The choice between the renders of a large chunk (csrc/tile_plan.h, the
 functions capi.cu and k_seg_decide use), built for the host: a chunk is
 rendered by tiles only when its (disc, tile) pairs are known to fit the pair
-list, whatever other buffers there are."""
+list, whatever other buffers there are.  And the order of a tile's discs: by
+octaves of the deposit scale, such that no deposit is lost on the FP32 sum of the
+ones before it."""
 import ctypes as C
 import itertools
+import math
 import os
 import subprocess
 
@@ -44,3 +47,17 @@ def test_no_chunk_overflows_the_pair_list(lib, n, nside):
             assert mode == 2
         else:
             assert mode == (1 if seg else 0), (tile, seg, pairs, cap)
+
+
+def test_no_deposit_is_lost_on_the_ones_before(lib):
+    """For every range of octaves: classes ascend with the octaves and there are
+    64 of them; with the discs of one class in any order, the smallest addend
+    (the class's smallest scale, times a weight of exp(-6)) is above half an ulp
+    of the largest total before it (a unit's discs at the class's largest scale)."""
+    for omax in range(256):
+        for omin in range(omax + 1):
+            c = [lib.cls(o, omax, omin) for o in range(omin, omax + 1)]
+            assert c[0] >= 0 and c[-1] == 63 and all(a <= b for a, b in zip(c, c[1:]))
+            width = max(c.count(k) for k in set(c))
+            least, total = math.exp(-6.0), lib.unit_max() * 2.0 ** width   # in the class's smallest scale
+            assert least > 2.0 ** -24 * total
