@@ -16,17 +16,13 @@
 #include <vector>
 
 #include "../../include/dmann.h"
+#include "dev_buf.h"
 #include "frame.h"
 #include "kernels.cuh"
 
 using namespace dmann;
 
 namespace {
-
-struct DevBuf {
-    void *p = nullptr;
-    size_t bytes = 0;
-};
 
 struct RingTables {
     double *z = nullptr, *st = nullptr, *theta = nullptr, *step = nullptr;
@@ -138,49 +134,45 @@ int block_bucket_min(const dmann_tuning &t) {
                         std::string(#call) + ": " + cudaGetErrorString(e_));                      \
     } while (0)
 
-// The compensated kernels' disc headers for n particles (comp_hdr_bytes()
-// each, with headroom for slowly growing chunks).  Optional: without them
-// the kernels compute each header themselves -- slower, the same results --
-// so a failed allocation is not an error.
-// Incremented by every (re)allocation of a context buffer: a captured batch
+// Changed by every allocation and release of a context buffer: a captured batch
 // graph holds buffer addresses, so a batch is recaptured after any.
 std::atomic<unsigned long long> g_alloc_gen{0};
 
-void reserve_headers(dmann_ctx *ctx, size_t n) {
-    const size_t bytes = comp_hdr_bytes() * (n > 0 ? n : 1);
-    if (ctx->w->chdr.bytes >= bytes) return;
-    if (ctx->w->chdr.p) cudaFree(ctx->w->chdr.p);
-    ctx->w->chdr.p = nullptr;
-    ctx->w->chdr.bytes = 0;
-    ++g_alloc_gen;
-    for (size_t want : {bytes + bytes / 8, bytes}) {
-        if (cudaMalloc(&ctx->w->chdr.p, want) == cudaSuccess) {
-            ctx->w->chdr.bytes = want;
-            return;
+struct CudaMem {
+    void *alloc(size_t bytes) {
+        void *p = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
         }
-        cudaGetLastError();
-        ctx->w->chdr.p = nullptr;
+        ++g_alloc_gen;
+        return p;
     }
+    void release(void *p) {   // (waits for the kernels in flight)
+        ++g_alloc_gen;
+        cudaFree(p);
+    }
+    size_t available() {
+        size_t free = 0, total = 0;
+        if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return free;
+    }
+};
+
+// An optional buffer: a failed allocation is not an error (the caller takes a
+// path that does without it).
+bool ensure_opt(DevBuf &b, size_t bytes) {
+    CudaMem m;
+    return grow(m, b, bytes);
 }
 
-// An optional buffer: grows like ensure() but a failed allocation is not an
-// error (the caller takes a path that does without it).
-bool ensure_opt(DevBuf &b, size_t bytes) {
-    if (b.bytes >= bytes) return true;
-    ++g_alloc_gen;
-    if (b.p) cudaFree(b.p);
-    b.p = nullptr;
-    b.bytes = 0;
-    for (size_t want : {bytes + bytes / 8, bytes}) {
-        if (cudaMalloc(&b.p, want) == cudaSuccess) {
-            b.bytes = want;
-            return true;
-        }
-        cudaGetLastError();
-        b.p = nullptr;
-    }
-    return false;
-}
+// The compensated kernels' disc headers for n particles (comp_hdr_bytes()
+// each).  Optional: without them the kernels compute each header themselves --
+// slower, the same results.
+void reserve_headers(dmann_ctx *ctx, size_t n) { ensure_opt(ctx->w->chdr, comp_hdr_bytes() * (n > 0 ? n : 1)); }
 
 // The plain form's scratch (2^25 doubles: 55,000 pixels' weights for each of
 // the 608 blocks of the block kernel; less for small maps) and, per Nside, its
@@ -227,29 +219,23 @@ CompHdr *headers_for(const dmann_ctx *ctx, size_t n) {
     return fits ? (CompHdr *)ctx->w->chdr.p : nullptr;
 }
 
-dmann_status ensure(dmann_ctx *ctx, DevBuf &b, size_t bytes) {
-    if (b.bytes >= bytes) return DMANN_OK;
-    ++g_alloc_gen;
-    if (b.p) {
-        cudaFree(b.p);
-        b.p = nullptr;
-        b.bytes = 0;
-    }
-    size_t want = bytes + bytes / 8;  // headroom for slowly growing chunks
-    cudaError_t e = cudaMalloc(&b.p, want);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        e = cudaMalloc(&b.p, bytes);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            b.p = nullptr;
-            return fail(ctx, DMANN_ERR_NOMEM,
-                        "device allocation of " + std::to_string(bytes) + " bytes failed");
-        }
-        want = bytes;
-    }
-    b.bytes = want;
-    return DMANN_OK;
+// The buffers that renders use where they have them.  Every call looks at them
+// after its required buffers are there, so these may take their place.
+std::vector<DevBuf *> optional_buffers(dmann_ctx *ctx) {
+    std::vector<DevBuf *> v;
+    for (Work &w : ctx->work)
+        for (DevBuf *b : {&w.tile_list, &w.tile_units, &w.tile_hist, &w.tile_base, &w.tile_hdr, &w.tile_gen,
+                          &w.seg_items, &w.seg_sorted, &w.seg_cls, &w.seg_first, &w.seg_nit, &w.seg_S, &w.seg_px,
+                          &w.plane32, &w.scratch, &w.chdr})
+            v.push_back(b);
+    return v;
+}
+
+// A required buffer; give_back: in place of the optional ones if need be.
+dmann_status ensure(dmann_ctx *ctx, DevBuf &b, size_t bytes, bool give_back = true) {
+    CudaMem m;
+    if (grow(m, b, bytes) || (give_back && grow_required(m, b, bytes, optional_buffers(ctx)))) return DMANN_OK;
+    return fail(ctx, DMANN_ERR_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes failed");
 }
 
 bool is_device_ptr(const void *p) {
@@ -756,15 +742,36 @@ size_t seg_capacity(size_t n) {
 // graph capture.
 bool have_opt(DevBuf &b, size_t bytes, bool grow) { return grow ? ensure_opt(b, bytes) : b.bytes >= bytes; }
 
-bool have_tile(dmann_ctx *ctx, size_t n, int nside, bool grow) {
+// slots: those of the pair list.
+bool have_tile(dmann_ctx *ctx, size_t n, int nside, bool grow, size_t &slots) {
     Work &w = *ctx->w;
     const size_t n1 = n > 0 ? n : 1, nt = (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
-    return have_opt(w.seg_S, 8 * n1, grow) && have_opt(w.seg_px, 8 * n1, grow) &&
-           have_opt(w.seg_cls, kSegBufBytes, grow) && have_opt(w.tile_gen, 4 * n1, grow) && have_opt(w.tile_hdr, sizeof(TileHdr) * n1, grow) &&
-           have_opt(w.tile_hist, kTileLists * nt * kTileClasses * sizeof(unsigned), grow) &&
-           have_opt(w.tile_base, kTileLists * nt * sizeof(long long), grow) &&
-           have_opt(w.tile_units, kTileLists * tile_unit_capacity(n, nside) * sizeof(TileUnit), grow) &&
-           have_opt(w.tile_list, 4 * tile_capacity(n, nside), grow);
+    struct {
+        DevBuf &b;
+        size_t bytes;
+    } fixed[] = {{w.seg_S, 8 * n1},
+                 {w.seg_px, 8 * n1},
+                 {w.seg_cls, kSegBufBytes},
+                 {w.tile_gen, 4 * n1},
+                 {w.tile_hdr, sizeof(TileHdr) * n1},
+                 {w.tile_hist, kTileLists * nt * kTileClasses * sizeof(unsigned)},
+                 {w.tile_base, kTileLists * nt * sizeof(long long)},
+                 {w.tile_units, kTileLists * tile_unit_capacity(tile_capacity(n, nside), nside) * sizeof(TileUnit)}};
+    if (grow) {
+        size_t beside = 0;
+        for (auto &f : fixed)
+            if (f.b.bytes < f.bytes) beside += f.bytes + f.bytes / 8;
+        CudaMem m;
+        grow_share(m, w.tile_list, 4 * tile_least(n, nside), 4 * tile_capacity(n, nside), beside);
+    }
+    slots = tile_slots(n, nside, w.tile_list.bytes / 4);
+    bool have = slots > 0;
+    for (auto &f : fixed) have = have && have_opt(f.b, f.bytes, grow);
+    if (!have && grow) {   // leave the room to the segments
+        CudaMem m;
+        for (DevBuf *b : {&w.tile_list, &w.tile_units, &w.tile_hist, &w.tile_base, &w.tile_hdr, &w.tile_gen}) drop(m, *b);
+    }
+    return have;
 }
 
 // (the FP32 plane is zeroed here, on the context's stream, when it is new)
@@ -792,9 +799,10 @@ bool may_be_large(size_t n, int nside, const dmann_tuning &tu) {
 
 bool reserve_large(dmann_ctx *ctx, size_t n, int nside, const dmann_tuning &tu) {
     if (!may_be_large(n, nside, tu)) return true;
-    const bool tile = tu.large_render != kLargeSegments && have_tile(ctx, n, nside, true);
+    size_t slots = 0;
+    const bool tile = tu.large_render != kLargeSegments && have_tile(ctx, n, nside, true, slots);
     const bool seg = tu.large_render != kLargeTiles;
-    return (tile && tile_always_fits(n, nside)) || (seg && have_seg(ctx, n, nside, true)) || tile;
+    return (tile && tile_always_fits(n, nside, slots)) || (seg && have_seg(ctx, n, nside, true)) || tile;
 }
 
 // The compensated form's block-class discs of a chunk that may be large:
@@ -815,8 +823,9 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     const int nside = ctx->g.nside;
     if (!da.chdr || !may_be_large(N, nside, tu)) return DMANN_OK;
     Work &w = *ctx->w;
-    const bool have_t = tu.large_render != kLargeSegments && have_tile(ctx, N, nside, grow);
-    const bool fits = tile_always_fits(N, nside), want_s = tu.large_render != kLargeTiles && !(have_t && fits);
+    size_t slots = 0;
+    const bool have_t = tu.large_render != kLargeSegments && have_tile(ctx, N, nside, grow, slots);
+    const bool fits = tile_always_fits(N, nside, slots), want_s = tu.large_render != kLargeTiles && !(have_t && fits);
     const auto [tile, seg, count] = plan_large(have_t, fits, want_s && have_seg(ctx, N, nside, grow));
     if (!tile && !seg) return DMANN_OK;
     cudaStream_t s = ctx->stream;
@@ -827,7 +836,7 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     sg.items = (int2 *)w.seg_items.p;
     sg.sorted = (int2 *)w.seg_sorted.p;
     sg.cap = seg ? (long long)seg_capacity(N) : 0;
-    sg.pair_cap = tile ? (long long)tile_capacity(N, nside) : 0;
+    sg.pair_cap = tile ? (long long)slots : 0;
     sg.cls = (int *)buf;
     sg.cls_px = (long long *)(buf + kSegClsBytes);
     sg.seg_next = (unsigned long long *)(buf + kSegClsBytes + kSegClsPxBytes);
@@ -849,7 +858,7 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     tg.hist = (unsigned *)w.tile_hist.p;
     tg.base = (long long *)w.tile_base.p;
     tg.units = (TileUnit *)w.tile_units.p;
-    tg.unit_cap = (long long)tile_unit_capacity(N, nside);
+    tg.unit_cap = (long long)tile_unit_capacity(slots, nside);
     tg.disc_S = sg.disc_S;
     tg.disc_px = sg.disc_px;
     tg.gen = (int *)w.tile_gen.p;
@@ -1221,12 +1230,16 @@ dmann_status dmann_render_batch(dmann_ctx *ctx, const float *x, const float *y, 
     for (int L = 0; L < lanes; L++) {
         ctx->w = &ctx->work[L];
         st = DMANN_OK;
-        if ((st = ensure(ctx, ctx->w->theta, 8 * n1)) || (st = ensure(ctx, ctx->w->phi, 8 * n1)) ||
-            (st = ensure(ctx, ctx->w->ar, 8 * n1)) || (st = ensure(ctx, ctx->w->flux, 8 * n1)) ||
-            (st = ensure(ctx, ctx->w->cpix, 4 * n1)) || (st = ensure(ctx, ctx->w->key, 4 * n1)) ||
-            (st = ensure(ctx, ctx->w->queue, 4 * n1)) || (st = ensure(ctx, ctx->w->hist, 4 * (size_t)kKeys)) ||
-            (st = ensure(ctx, ctx->w->ctr, 8 * C_COUNT)) || (st = ensure(ctx, ctx->w->fsum, 8)) ||
-            (st = ensure(ctx, ctx->w->acc, 8 * Pmax))) {
+        const struct {
+            DevBuf &b;
+            size_t bytes;
+        } need[] = {{ctx->w->theta, 8 * n1}, {ctx->w->phi, 8 * n1}, {ctx->w->ar, 8 * n1}, {ctx->w->flux, 8 * n1},
+                    {ctx->w->cpix, 4 * n1}, {ctx->w->key, 4 * n1}, {ctx->w->queue, 4 * n1},
+                    {ctx->w->hist, 4 * (size_t)kKeys}, {ctx->w->ctr, 8 * C_COUNT}, {ctx->w->fsum, 8},
+                    {ctx->w->acc, 8 * Pmax}};
+        for (auto &f : need)   // (the second lane does not take the first one's optional buffers)
+            if (st == DMANN_OK) st = ensure(ctx, f.b, f.bytes, L == 0);
+        if (st != DMANN_OK) {
             ctx->w = &ctx->work[0];
             if (L == 0) return st;
             lanes = 1;   // no room for a second workspace: one lane

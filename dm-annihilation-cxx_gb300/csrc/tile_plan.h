@@ -35,18 +35,24 @@ DMANN_HD inline int tile_class(int oct, int omax, int omin) {
 inline size_t tile_pairs_bound(size_t n, int nside) {
     return (n > 0 ? n : 1) * (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
 }
-// Pair list slots of the tiled render: every disc in every tile where that
-// is little (then no chunk can exceed it), else 96 per particle and 2^24 (a
-// disc of the 16M set at Nside 2048 touches 33 tiles, one of the 134M set at
-// Nside 4096 about 55; chunks with more pairs are segmented).
+// Pair list slots that the tiled render asks for: every disc in every tile
+// where that is little (then no chunk can exceed it), else 96 per particle and
+// 2^24 (a disc of the 16M set at Nside 2048 touches 33 tiles, one of the 134M set
+// at Nside 4096 about 55; chunks with more pairs are segmented).
 inline size_t tile_capacity(size_t n, int nside) {
     return std::min(tile_pairs_bound(n, nside), 96 * n + ((size_t)1 << 24));
 }
-inline size_t tile_unit_capacity(size_t n, int nside) {
-    return tile_capacity(n, nside) / kUnitMax + 2 * (size_t)kUnitTarget +
-           (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
+// Fewer are of no use, and more than the list holds are not used.
+inline size_t tile_least(size_t n, int nside) {
+    return std::min(tile_pairs_bound(n, nside), 8 * n + ((size_t)1 << 16));
 }
-inline bool tile_always_fits(size_t n, int nside) { return tile_capacity(n, nside) == tile_pairs_bound(n, nside); }
+inline size_t tile_slots(size_t n, int nside, size_t list) {
+    return list >= tile_least(n, nside) ? std::min(list, tile_capacity(n, nside)) : 0;
+}
+inline size_t tile_unit_capacity(size_t slots, int nside) {
+    return slots / kUnitMax + 2 * (size_t)kUnitTarget + (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
+}
+inline bool tile_always_fits(size_t n, int nside, size_t slots) { return slots >= tile_pairs_bound(n, nside); }
 
 // dmann_tuning.large_render
 enum { kLargeAny = 1, kLargeTiles = 2, kLargeSegments = 3 };

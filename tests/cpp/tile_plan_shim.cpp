@@ -7,7 +7,8 @@ using namespace dmann;
 extern "C" {
 long long pairs_bound(long long n, int nside) { return (long long)tile_pairs_bound(n, nside); }
 long long capacity(long long n, int nside) { return (long long)tile_capacity(n, nside); }
-int always_fits(long long n, int nside) { return tile_always_fits(n, nside); }
+long long slots(long long n, int nside, long long list) { return (long long)tile_slots(n, nside, list); }
+int always_fits(long long n, int nside) { return tile_always_fits(n, nside, tile_capacity(n, nside)); }
 // bit 0 tiles, 1 segments, 2 the pair count
 int plan(int have_tile, int fits, int have_seg) {
     const LargePlan p = plan_large(have_tile, fits, have_seg);
