@@ -28,7 +28,7 @@ struct RingTables {
     double *z = nullptr, *st = nullptr, *theta = nullptr, *step = nullptr;
     float *st32 = nullptr, *step32 = nullptr;
     float2 *th2 = nullptr;
-    double2 *trig_belt = nullptr, *trig_cap = nullptr;   // the plain form's, built on first use
+    DevBuf trig_belt, trig_cap;   // the plain form's, built on first use (double2)
 };
 
 }  // namespace
@@ -181,27 +181,23 @@ void reserve_plain(dmann_ctx *ctx, int nside) {
     const size_t npix = 12 * (size_t)nside * (size_t)nside;
     ensure_opt(ctx->w->scratch, 8 * std::min((size_t)1 << 25, 32768 * npix));
     auto it = ctx->rings.find(nside);
-    if (it == ctx->rings.end() || it->second.trig_belt) return;
+    if (it == ctx->rings.end() || it->second.trig_belt.p) return;
     RingTables &t = it->second;
-    const size_t cap = 2 * (size_t)nside * (nside - 1);
-    if (cudaMalloc(&t.trig_belt, sizeof(double2) * 8 * nside) != cudaSuccess) {
-        cudaGetLastError();
-        t.trig_belt = nullptr;
-        return;
-    }
-    // a cap's table up to Nside 1448 (64 MB)
-    if (cap > 0 && sizeof(double2) * cap <= ((size_t)64 << 20) &&
-        cudaMalloc(&t.trig_cap, sizeof(double2) * cap) != cudaSuccess) {
-        cudaGetLastError();
-        t.trig_cap = nullptr;
-    }
+    size_t held = 0;
+    for (auto &kv : ctx->rings) held += kv.second.trig_cap.bytes;
+    CudaMem m;
+    auto take = [&m](DevBuf &b, size_t bytes) {
+        if (bytes > 0 && (b.p = m.alloc(bytes))) b.bytes = bytes;
+        return b.p != nullptr;
+    };
+    if (!take(t.trig_belt, sizeof(double2) * 8 * nside)) return;
+    take(t.trig_cap, trig_cap_bytes(nside, held));
     // the tables outlive this map and its stream: complete before any use
-    if (launch_trig(nside, (double)(nside << 1) * (4.0 / (double)npix), t.trig_belt, t.trig_cap, ctx->stream) !=
-            cudaSuccess ||
+    if (launch_trig(nside, (double)(nside << 1) * (4.0 / (double)npix), (double2 *)t.trig_belt.p,
+                    (double2 *)t.trig_cap.p, ctx->stream) != cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-        cudaFree(t.trig_belt);
-        if (t.trig_cap) cudaFree(t.trig_cap);
-        t.trig_belt = t.trig_cap = nullptr;
+        drop(m, t.trig_belt);
+        drop(m, t.trig_cap);
     }
 }
 
@@ -210,8 +206,8 @@ void plain_args(const dmann_ctx *ctx, int nside, DiscArgs &da) {
     da.scratch_total = (long long)(ctx->w->scratch.bytes / 8);
     auto it = ctx->rings.find(nside);
     if (it == ctx->rings.end()) return;
-    da.trig_belt = it->second.trig_belt;
-    da.trig_cap = it->second.trig_cap;
+    da.trig_belt = (const double2 *)it->second.trig_belt.p;
+    da.trig_cap = (const double2 *)it->second.trig_cap.p;
 }
 
 CompHdr *headers_for(const dmann_ctx *ctx, size_t n) {
@@ -228,6 +224,8 @@ std::vector<DevBuf *> optional_buffers(dmann_ctx *ctx) {
                           &w.seg_items, &w.seg_sorted, &w.seg_cls, &w.seg_first, &w.seg_nit, &w.seg_S, &w.seg_px,
                           &w.plane32, &w.scratch, &w.chdr})
             v.push_back(b);
+    for (auto &kv : ctx->rings)
+        for (DevBuf *b : {&kv.second.trig_belt, &kv.second.trig_cap}) v.push_back(b);
     return v;
 }
 
@@ -457,8 +455,8 @@ void dmann_destroy(dmann_ctx *ctx) {
         cudaFree(kv.second.st32);
         cudaFree(kv.second.step32);
         cudaFree(kv.second.th2);
-        if (kv.second.trig_belt) cudaFree(kv.second.trig_belt);
-        if (kv.second.trig_cap) cudaFree(kv.second.trig_cap);
+        if (kv.second.trig_belt.p) cudaFree(kv.second.trig_belt.p);
+        if (kv.second.trig_cap.p) cudaFree(kv.second.trig_cap.p);
     }
     if (ctx->h_ctr) cudaFreeHost(ctx->h_ctr);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);

@@ -62,4 +62,12 @@ size_t grow_share(M &m, DevBuf &b, size_t least, size_t most, size_t beside) {
     return b.bytes;
 }
 
+// The plain form's azimuth table of a cap at one Nside, in bytes: 64 MB at most
+// (Nside 1448), and none where a context that renders at many Nside would hold
+// more than 256 MB of them (`held` so far); its maps compute the azimuths then.
+inline size_t trig_cap_bytes(int nside, size_t held) {
+    const size_t bytes = 16 * 2 * (size_t)nside * (size_t)(nside - 1);
+    return bytes <= ((size_t)64 << 20) && held + bytes <= ((size_t)256 << 20) ? bytes : 0;
+}
+
 }  // namespace dmann

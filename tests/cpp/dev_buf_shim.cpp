@@ -51,5 +51,6 @@ void free_buf(int b) { drop(mem, bufs[b]); }
 long long held(int b) { return (long long)bufs[b].bytes; }
 long long used() { return (long long)mem.used; }
 long long changes() { return (long long)mem.changes; }
+long long trig_cap(int nside, long long held) { return (long long)trig_cap_bytes(nside, (size_t)held); }
 long long calls() { return (long long)mem.calls; }
 }

@@ -66,3 +66,13 @@ def test_a_share_is_kept_while_the_free_memory_moves(lib):
         assert lib.share(0, 100, 100000, 0) == first and lib.changes() == m
     assert lib.share(0, first + 1, 100000, 0) == 0   # fewer than it takes now
     assert lib.changes() >= n
+
+
+def test_azimuth_tables_are_bounded(lib):
+    """A context that renders the plain form at every Nside."""
+    lib.trig_cap.argtypes, lib.trig_cap.restype = [C.c_int, C.c_longlong], C.c_longlong
+    assert all(lib.trig_cap(n, 0) == 32 * n * (n - 1) for n in (1, 64, 512, 1024, 1448))
+    held = 0
+    for nside in range(1, 8193):
+        held += lib.trig_cap(nside, held)
+    assert held <= 256 << 20
