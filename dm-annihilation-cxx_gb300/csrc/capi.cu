@@ -754,7 +754,7 @@ bool have_tile(dmann_ctx *ctx, size_t n, int nside, bool grow, size_t &slots) {
                  {w.tile_hdr, sizeof(TileHdr) * n1},
                  {w.tile_hist, kTileLists * nt * kTileClasses * sizeof(unsigned)},
                  {w.tile_base, kTileLists * nt * sizeof(long long)},
-                 {w.tile_units, kTileLists * tile_unit_capacity(tile_capacity(n, nside), nside) * sizeof(TileUnit)}};
+                 {w.tile_units, tile_unit_capacity(tile_capacity(n, nside), nside) * sizeof(TileUnit)}};
     if (grow) {
         size_t beside = 0;
         for (auto &f : fixed)
@@ -856,7 +856,6 @@ dmann_status render_large(dmann_ctx *ctx, const DiscArgs &da, const dmann_tuning
     tg.hist = (unsigned *)w.tile_hist.p;
     tg.base = (long long *)w.tile_base.p;
     tg.units = (TileUnit *)w.tile_units.p;
-    tg.unit_cap = (long long)tile_unit_capacity(slots, nside);
     tg.disc_S = sg.disc_S;
     tg.disc_px = sg.disc_px;
     tg.gen = (int *)w.tile_gen.p;

@@ -867,6 +867,13 @@ __global__ void __launch_bounds__(256) k_tile_pairs(DiscArgs a, TileArgs tg) {
         for (int k = 0; k < kTileLists; k++) count(C_TILE_PAIRS + k, list[k]);
 }
 
+// The first unit of list k.
+__device__ __forceinline__ long long first_unit(const DiscArgs &a, const TileArgs &tg, int k) {
+    long long f = 0;
+    for (int j = 0; j < k; j++) f += tile_units_of(a.ctr[C_TILE_PAIRS + j], (long long)tg.nstrips * tg.ncol);
+    return f;
+}
+
 // Each tile's range of the pair list and its units: a warp per tile.
 __global__ void __launch_bounds__(256) k_tile_plan(DiscArgs a, TileArgs tg) {
     if (tg.ctl[0] != 2) return;
@@ -874,11 +881,6 @@ __global__ void __launch_bounds__(256) k_tile_plan(DiscArgs a, TileArgs tg) {
     const int NT = tg.nstrips * tg.ncol;
     const int nt = kTileLists * NT;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    // enough units of each list to spread over the GPU, long enough to pay for
-    // their flush
-    auto unit_len = [&](int k) {
-        return (int)min((long long)kUnitMax, max((long long)kUnitMin, a.ctr[C_TILE_PAIRS + k] / kUnitTarget));
-    };
     for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nw) {
         static_assert(kCls == 64, "two octaves per lane");
         uint2 *hp = reinterpret_cast<uint2 *>(tg.hist + ((size_t)t << kClsBits)) + lane;
@@ -888,7 +890,7 @@ __global__ void __launch_bounds__(256) k_tile_plan(DiscArgs a, TileArgs tg) {
         if (total == 0) continue;
         *hp = make_uint2((unsigned)ex, (unsigned)ex + v.x);
         const int which = t / NT;
-        const int ulen = unit_len(which), nu = (total + ulen - 1) / ulen;
+        const int ulen = tile_unit_len(a.ctr[C_TILE_PAIRS + which]), nu = (total + ulen - 1) / ulen;
         long long b = 0, u = 0;
         if (lane == 0) {
             b = (long long)atomicAdd((unsigned long long *)(a.ctr + C_TILE_CURSOR), (unsigned long long)total);
@@ -898,7 +900,7 @@ __global__ void __launch_bounds__(256) k_tile_plan(DiscArgs a, TileArgs tg) {
         b = __shfl_sync(0xffffffffu, b, 0);
         u = __shfl_sync(0xffffffffu, u, 0);
         const int per = (total + nu - 1) / nu;
-        TileUnit *out = tg.units + which * tg.unit_cap + u;
+        TileUnit *out = tg.units + first_unit(a, tg, which) + u;
         for (int k = lane; k < nu; k += 32) {
             TileUnit w;
             w.start = b + (long long)k * per;
@@ -1117,7 +1119,7 @@ __device__ __forceinline__ bool claim_unit(const DiscArgs &a, const TileArgs &tg
     if ((threadIdx.x & 31) == 0) u = (long long)atomicAdd((unsigned long long *)(a.ctr + C_UNEXT + which), 1ull);
     u = __shfl_sync(0xffffffffu, u, 0);
     if (u >= a.ctr[C_UNITS + which]) return false;
-    un = tg.units[which * tg.unit_cap + u];
+    un = tg.units[first_unit(a, tg, which) + u];
     return true;
 }
 
@@ -1213,13 +1215,13 @@ __global__ void __launch_bounds__(kGenWarps * 32)
     __shared__ float2 tile[kGenWarps][32 * kRow];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float2 *const my = tile[w] + lane * kRow;
-    const long long halves = 2 * a.ctr[C_UNITS + 3];
+    const long long halves = 2 * a.ctr[C_UNITS + 3], first = first_unit(a, tg, 3);
     for (;;) {
         long long u = 0;
         if (lane == 0) u = (long long)atomicAdd((unsigned long long *)(a.ctr + C_UNEXT + 3), 1ull);
         u = __shfl_sync(0xffffffffu, u, 0);
         if (u >= halves) break;
-        const TileUnit un = tg.units[3 * tg.unit_cap + (u >> 1)];
+        const TileUnit un = tg.units[first + (u >> 1)];
         const int strip = un.tile / tg.ncol, base = (un.tile - strip * tg.ncol) * kTileW + (int)(u & 1) * kPxW;
         const int ring = min(strip * kTileR + 1 + lane, a.g.nrings);
         const bool own = strip * kTileR + 1 + lane <= a.g.nrings;

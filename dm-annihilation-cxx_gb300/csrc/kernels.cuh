@@ -181,8 +181,7 @@ struct TileArgs {
     unsigned *list;           // the pairs' discs, tile by tile
     unsigned *hist;           // [kTileLists][tiles][kTileClasses]: pairs per octave, then list slots
     long long *base;          // [kTileLists][tiles]: each tile's first list slot
-    TileUnit *units;          // [kTileLists][unit_cap]
-    long long unit_cap;
+    TileUnit *units;          // of each list, one behind the other
     double *disc_S;           // per block-class disc, as SegArgs
     long long *disc_px;
     int *gen;                 // queue slots of the giant discs (C_GEN, from the front) and of the long

@@ -11,9 +11,13 @@ namespace dmann {
 
 // A tile is kTileR rings by kTileW in-ring pixel indices, a unit up to
 // kUnitMax discs of its list (fewer while the chunk has less than kUnitTarget
-// units of more than kUnitMin).
+// units of more than kUnitMin).  A unit's FP32 sums are rounded by 1.7e-8 of their
+// total at each addition, so a pixel of M deposits is off by 1.7e-8 kUnitMax /
+// sqrt(3 M): with units of 512 that was most of the error of a map's bright
+// regions (7e-8 of 1M particles at Nside 512, 4.8e-8 with 128), and their flush
+// is as little of the time either way.
 constexpr int kTileR = 32, kTileW = 64;
-constexpr int kUnitMin = 32, kUnitMax = 512, kUnitTarget = 16384;
+constexpr int kUnitMin = 32, kUnitMax = 128, kUnitTarget = 16384;
 constexpr int kTileClasses = 64;
 constexpr int kTileLists = 4;
 
@@ -49,8 +53,15 @@ inline size_t tile_least(size_t n, int nside) {
 inline size_t tile_slots(size_t n, int nside, size_t list) {
     return list >= tile_least(n, nside) ? std::min(list, tile_capacity(n, nside)) : 0;
 }
+// Discs per unit of a list of `pairs`, and the units it makes at most on nt tiles.
+DMANN_HD inline int tile_unit_len(long long pairs) {
+    const long long k = pairs / kUnitTarget;
+    return (int)(k < kUnitMin ? kUnitMin : k > kUnitMax ? kUnitMax : k);
+}
+DMANN_HD inline long long tile_units_of(long long pairs, long long nt) { return pairs / tile_unit_len(pairs) + nt; }
+// The units of all lists, one behind the other.
 inline size_t tile_unit_capacity(size_t slots, int nside) {
-    return slots / kUnitMax + 2 * (size_t)kUnitTarget + (size_t)tile_strips(nside) * (size_t)tile_cols(nside);
+    return slots / kUnitMax + kTileLists * (2 * (size_t)kUnitTarget + (size_t)tile_strips(nside) * (size_t)tile_cols(nside));
 }
 inline bool tile_always_fits(size_t n, int nside, size_t slots) { return slots >= tile_pairs_bound(n, nside); }
 

@@ -19,5 +19,8 @@ int mode(long long est, long long min_est, long long blocks, long long pairs, lo
     return large_mode(est, min_est, blocks, pairs, pair_cap, items, item_cap);
 }
 int cls(int oct, int omax, int omin) { return tile_class(oct, omax, omin); }
+int unit_len(long long pairs) { return tile_unit_len(pairs); }
+long long units_of(long long pairs, long long nt) { return tile_units_of(pairs, nt); }
+long long unit_capacity(long long slots, int nside) { return (long long)tile_unit_capacity(slots, nside); }
 int unit_max() { return kUnitMax; }
 }

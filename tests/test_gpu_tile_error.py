@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 
 import annmap
+from annmap import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +45,23 @@ def test_pixel_errors(rend, nside, n, lo, hi):
         err[large] = np.linalg.norm(got - ref) / np.linalg.norm(ref)
     print("error", err)
     assert err[TILES] <= 1.05 * err[SEGMENTS]
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_dense_map(rend, seed):
+    """A third of a million particles of a halo of four: thousands of deposits in
+    the bright pixels, whose FP32 sums (of at most 128 discs, tile_plan.h) are
+    then the error; 10 % for the luck of the brightest few."""
+    n, nside = 346889, 742
+    P = synth.nfw_halo(n, seed=seed, n_total=1 << 22, near_observer=20)
+    with annmap.Renderer(0) as r:
+        r.set_params(annmap.Parameters.for_synthetic(P, nside))
+        ref = r.render(P.as_dict(), nside, PLAIN)
+        err = {}
+        for large in (TILES, SEGMENTS):
+            r.set_tuning(large_render=large)
+            got = r.render(P.as_dict(), nside, COMP)
+            assert r.stats()["pass2_ms"] > 0.0
+            err[large] = np.linalg.norm(got - ref) / np.linalg.norm(ref)
+    print("error", err)
+    assert err[TILES] <= 1.1 * err[SEGMENTS]

@@ -61,3 +61,25 @@ def test_no_deposit_is_lost_on_the_ones_before(lib):
             width = max(c.count(k) for k in set(c))
             least, total = math.exp(-6.0), lib.unit_max() * 2.0 ** width   # in the class's smallest scale
             assert least > 2.0 ** -24 * total
+
+
+def test_the_units_of_all_lists_fit(lib):
+    """The lists' units, one behind the other, however the pairs are dealt to the
+    four lists and to the tiles (one pair in every tile but one makes the most)."""
+    L = C.c_longlong
+    lib.units_of.argtypes, lib.units_of.restype = [L, L], L
+    lib.unit_capacity.argtypes, lib.unit_capacity.restype = [L, C.c_int], L
+    lib.unit_len.argtypes = [L]
+    for nside in (64, 1024, 4096):
+        nt = ((4 * nside + 30) // 32) * ((4 * nside + 63) // 64)
+        for slots in (1, 1000, 1 << 19, 3 << 20, 1 << 24, 1 << 31):
+            for split in ((1, 0, 0, 0), (0.25, 0.25, 0.25, 0.25), (0.7, 0.1, 0.1, 0.1), (0.97, 0.01, 0.01, 0.01)):
+                pairs = [int(slots * f) for f in split]
+                room = [lib.units_of(p, nt) for p in pairs]
+                assert sum(room) <= lib.unit_capacity(slots, nside)
+                for p, have in zip(pairs, room):
+                    n = lib.unit_len(p)
+                    assert 32 <= n <= lib.unit_max()
+                    spread = min(p, nt)               # tiles with a pair
+                    most = (spread - 1 + (p - spread + 1 + n - 1) // n) if p else 0
+                    assert most <= have
