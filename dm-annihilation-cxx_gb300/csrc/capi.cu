@@ -34,7 +34,7 @@ struct RingTables {
 }  // namespace
 
 // One map's device work: the prep outputs, the queue, the counters and
-// accumulation planes, the disc headers and the segmented render's buffers.
+// accumulation planes, the disc headers and the two large renders' buffers.
 // A context renders with work[0]; a batch of device maps uses both, one
 // observer on each at a time.
 struct Work {
@@ -44,9 +44,9 @@ struct Work {
     // weight sums and pixel counts, and the FP32 deposit plane
     DevBuf seg_items, seg_sorted, seg_cls, seg_first, seg_nit, seg_S, seg_px, plane32;
     bool plane_clean = false;   // plane32 is all zero (every segment's flush leaves it so)
-    // tiled render (disc_tile.cu): the pair list, its histogram and ranges,
-    // the work units, the general discs
     DevBuf scratch;           // plain form: the weights of the discs in work
+    // tiled render (disc_tile.cu): the disc headers, the pair list, its
+    // histogram and ranges, the work units, the giant and the long discs
     DevBuf tile_hdr, tile_list, tile_hist, tile_base, tile_units, tile_gen;
 };
 
@@ -56,7 +56,7 @@ struct dmann_ctx {
     cudaStream_t own = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evd0 = nullptr, evdm = nullptr, evd1 = nullptr;
-    cudaEvent_t evp1 = nullptr;   // end of the segmented render's pass 1
+    cudaEvent_t evp1 = nullptr;   // end of a large render's pass 1
     bool disc_timed = false, seg_timed = false;
     bool have_frame = false, have_units = false;
     double rot[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
@@ -1242,7 +1242,7 @@ dmann_status dmann_render_batch(dmann_ctx *ctx, const float *x, const float *y, 
             lanes = 1;   // no room for a second workspace: one lane
             break;
         }
-        // before any capture: the disc headers and the segmented render's
+        // before any capture: the disc headers and the large renders'
         // buffers (the render checks them again and allocates nothing when
         // they fit)
         if (precision == DMANN_COMP_F32) {

@@ -141,7 +141,7 @@ constexpr int kWPB = 8, kRCHW = 64;    // warp kernel
 // rings staged per chunk, MINB resident blocks per SM -- every shape fills
 // the SM with 2048 threads (fewer, with more registers each, measured slower)
 // and about 200 KB of staged runs.  The autotuner picks the shape.  Returns
-// at once when the segmented render took the block class (*a.block_skip).
+// at once when a large chunk's render took the block class (*a.block_skip).
 template <int BT, int RCH, int MINB>
 __global__ void __launch_bounds__(BT, MINB) k_comp_block(DiscArgs a) {
     if (a.block_skip && *a.block_skip) return;

@@ -13,9 +13,11 @@
 // one FP64 reduction per pixel for up to kUnitMax discs.
 //
 // Sequence (one stream, nothing waits for the host):
-//   k_tile_total    (disc, tile) pairs of the chunk, for its mode
-//   k_tile_norm     weight sums S of the discs; k_tile_norm_giant
-//                   of the largest
+//   k_tile_hdr      a short header per disc; the giants and the long discs
+//   k_tile_pairs<0> (disc, tile) pairs of the chunk, for its mode (where they
+//                   could exceed the list)
+//   k_tile_norm     weight sums S of the discs; k_tile_norm_giant of the
+//                   giants, the largest and those that carry the map's flux
 //   k_tile_fin      F = flux / S per disc, discs of fewer than two pixels
 //   k_tile_pairs<1> pairs per (tile, octave of F)
 //   k_tile_plan     each tile's range of the pair list, its octaves in
@@ -73,12 +75,13 @@ constexpr double kGiantR = 2.2;
 // sum of flux bounds nothing.)
 constexpr int kShare = 256, kShareMax = 1024;
 
-// The y^4 term is at most 2.7e-8 in the exponent of 2 for half azimuth offsets
-// x below 0.1 rad (y = x^2) and the three-term asin^2 tier (h < 4e-3): a ninth
-// of the exponent's FP32 rounding.  sin R / sin theta0 = sin 2x at x = 0.1.
-// Without it the 16M workload takes 604 ms instead of 632; the maps' error
-// against the FP64 form is the same (Nside 512: 4.8e-8 with, 5.5e-8 without;
-// 2048: 8.1e-8 and 8.0e-8, 1.06e-7 and 1.06e-7).
+// Half azimuth offsets x below 0.1 rad (sin R / sin theta0 = sin 2x) of the
+// three-term asin^2 tier (h < 4e-3) do without the y^4 term (y = x^2): up to 6e-8
+// in the exponent of 2, most of it the share of h^3, which that of h^4, beyond the
+// three terms, would cancel.  With it a map of 1M particles at Nside 512 is
+// 1.17e-7 from the FP64 form instead of 8.9e-8, one of 200k at Nside 400 6.4e-8
+// instead of 3.9e-8 (units of 512 discs), and the 16M workload took 632 ms
+// instead of 604.
 constexpr float kPoly3Sin = 0.1987f;
 
 constexpr int kLongRings = 256;   // general discs of more are summed by several warps
@@ -270,7 +273,8 @@ __device__ __forceinline__ float2 ex2_2(float2 t) { return make_float2(ex2_appro
 // of 1/16, one of 32 dealt to the lanes anew for each disc, and its sum is
 // scaled back: the nodes then see the function's local average, as the
 // pixels do, but for 1.4e-9 (the mean over 300 discs of each of several radii
-// and Nside).
+// and Nside).  Sets of thousands of discs of one kind and size are left with
+// -5e-10 to 6e-10 of their flux (Nside 64 to 1024).
 constexpr float kEx2Bias = -1.4e-9f;
 
 struct Dither {

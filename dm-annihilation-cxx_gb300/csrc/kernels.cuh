@@ -22,10 +22,10 @@ constexpr int kKeys = kBuckets * kCells;
 
 // Segmented render (disc_seg.cu; its constants and segment plan are in
 // seg_plan.h).  The plan is made on the device; each chunk launches
-// kSegSlots deposit/flush pairs, the unused ones return at once.  Chunks
-// whose estimated deposits are below 2^seg_min_deposits_log2 (a tunable), or
-// whose work items exceed the item buffers, deposit in FP64 with the per-disc
-// kernels.
+// kSegSlots deposit/flush pairs, the unused ones return at once.  It takes the
+// chunks whose (disc, tile) pairs the tiled render's list does not hold; those
+// below 2^seg_min_deposits_log2 estimated deposits (a tunable), or with more
+// work items than the item buffers hold, deposit in FP64 with the per-disc kernels.
 // The segment buffer, zeroed per chunk: cls, cls_px, seg_next, spans, ctl.
 constexpr size_t kSegClsBytes = 2 * 4 * kClasses;
 constexpr size_t kSegClsPxBytes = 8 * kClasses;
@@ -120,7 +120,7 @@ struct DiscArgs {
     // launch; null computes each header inside the disc kernels instead
     CompHdr *chdr = nullptr;
     // compensated block kernel: returns at once when *block_skip != 0 (the
-    // segmented render took the chunk's block class); null = never
+    // tiled or the segmented render took the chunk's block class); null = never
     const int *block_skip = nullptr;
     // plain form: FP64 scratch for the weights of the discs in work (doubles;
     // scratch_len per group of threads, set by the launch), and (sin, cos) of
@@ -144,7 +144,7 @@ struct SegArgs {
     unsigned long long *seg_next;   // [kSegSlots]: items claimed by each segment
     SegSpan *spans;           // [kSegSlots]: the segment plan
     int *ctl;                 // [0] mode (0 per-disc kernels, 1 segmented, 2 tiled), [1] segments
-    long long min_est;        // estimated deposits from which the chunk is segmented
+    long long min_est;        // estimated deposits from which the chunk is tiled or segmented
     long long budget;         // deposits per segment before the plan splits an octave
     long long *disc_first;    // per block-class disc: its first item
     int *disc_nitems;         //   its item count
