@@ -804,47 +804,79 @@ __device__ inline void strip_cols(const DiscArgs &a, const TileHdr &h, int s, in
     c1 = max(c0, col_hi(hi));
 }
 
-constexpr int kPairLanes = 8;   // lanes (strips at a time) per disc
+constexpr int kPairLanes = 8;    // lanes (strips at a time) per disc
+constexpr int kWideParts = 64, kWideStrips = 96;   // warps of a giant or long disc of more strips than that
 
 // MODE 0: the chunk's pairs, before S is known (for its mode; at least those
 // of mode 1, which leaves out discs with nothing to deposit); 1: pairs per
 // (tile, octave); 2: the pair list.  Bound by the latency of the slot atomics:
-// mode 2 takes 1.3 ms with four on their way, 2.7 ms one at a time.
+// mode 2 takes 1.3 ms with four on their way, 2.7 ms one at a time.  The tallest
+// of the giants and long discs have their strips dealt to kWideParts warps, a
+// column per lane: one disc over the whole map at Nside 8192, half a million
+// pairs, kept its 8 lanes busy for 11 ms.  (With every long disc dealt out the
+// three modes take 1.16 ms of 1M particles at Nside 512 instead of 0.48.)
 template <int MODE>
 __global__ void __launch_bounds__(256) k_tile_pairs(DiscArgs a, TileArgs tg) {
     if (MODE != 0 && tg.ctl[0] != 2) return;
     const long long nblk = a.ctr[C_ADD_BLOCK];
-    const int sl = threadIdx.x % kPairLanes;
-    const long long stride = (long long)gridDim.x * blockDim.x / kPairLanes;
+    const int sl = threadIdx.x % kPairLanes, lane = threadIdx.x & 31;
+    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long threads = (long long)gridDim.x * blockDim.x;
     const int *const oc = reinterpret_cast<const int *>(a.ctr + C_OCT);
     const int omax = MODE ? oc[0] : 0, omin = MODE ? 255 - oc[1] : 0;
     const int NT = tg.nstrips * tg.ncol;
     long long total = 0, list[kTileLists] = {};
-    for (long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kPairLanes; q < nblk; q += stride) {
-        TileHdr h = tg.hdr[q];
-        int cls = 0;
-        if (MODE) {
-            const float F = h.F;
-            if (F == 0.0f) continue;   // nothing to deposit (weights are >= exp(-6))
-            cls = tile_class((int)((__float_as_uint(F) >> 23) & 255), omax, omin);
-        }
+    // a disc's class, negative with nothing to deposit (weights are >= exp(-6))
+    auto class_of = [&](const TileHdr &h) {
+        if (MODE == 0) return 0;
+        return h.F == 0.0f ? -1 : tile_class((int)((__float_as_uint(h.F) >> 23) & 255), omax, omin);
+    };
+    auto list_of = [](const TileHdr &h, int nlo) {
         const int kind = h.flags & kKindMask;
+        return kind <= K_POLY ? kind : kind == K_GEN && nlo >= kFineNr ? 2 : 3;
+    };
+    auto tally = [&](int which, int np) {
+        if (MODE == 0) total += np;
+#pragma unroll
+        for (int k = 0; k < kTileLists; k++) list[k] += which == k ? np : 0;
+    };
+    auto wide = [](const TileHdr &h) {
+        return ((h.flags & kKindMask) == K_GIANT || (h.flags & kFlagLong)) && h.r_last - h.r_first >= kWideStrips * kTileR;
+    };
+    const long long ngiant = a.ctr[C_GEN];
+    const long long nwide = tg.nstrips > kWideStrips ? (ngiant + tg.ctl[3]) * kWideParts : 0;
+    for (long long t = tid / 32; t < nwide; t += threads / 32) {
+        const long long k = t / kWideParts;
+        const int q = tg.gen[k < ngiant ? k : nblk - 1 - (k - ngiant)];
+        const TileHdr h = tg.hdr[q];
+        const int cls = class_of(h);
+        if (cls < 0 || !wide(h)) continue;
+        const int s1 = (h.r_last - 1) / kTileR;
+        for (int s = (h.r_first - 1) / kTileR + (int)(t % kWideParts); s <= s1; s += kWideParts) {
+            int nlo, c0, c1, c2, c3;
+            strip_cols(a, h, s, nlo, c0, c1, c2, c3);
+            const int n0 = c1 - c0 + 1, np = n0 + max(0, c3 - c2 + 1), which = list_of(h, nlo);
+            if (lane == 0) tally(which, np);
+            if (MODE == 0) continue;
+            for (int i = lane; i < np; i += 32) {
+                const int tile = which * NT + s * tg.ncol + (i < n0 ? c0 + i : c2 + (i - n0));
+                const unsigned slot = atomicAdd(tg.hist + ((size_t)tile << kClsBits) + cls, 1u);
+                if (MODE == 2) tg.list[tg.base[tile] + slot] = (unsigned)q;
+            }
+        }
+    }
+    for (long long q = tid / kPairLanes; q < nblk; q += threads / kPairLanes) {
+        TileHdr h = tg.hdr[q];
+        const int cls = class_of(h);
+        if (cls < 0 || wide(h)) continue;
         const int s1 = h.r_last >= h.r_first ? (h.r_last - 1) / kTileR : -1;
         for (int s = (h.r_first - 1) / kTileR + sl; s <= s1; s += kPairLanes) {
             int nlo, c0, c1, c2, c3;
             strip_cols(a, h, s, nlo, c0, c1, c2, c3);
-            const int np = (c1 - c0 + 1) + max(0, c3 - c2 + 1);
-            if (MODE == 0) {
-                total += np;
-                continue;
-            }
-            const int which = kind <= K_POLY ? kind : kind == K_GEN && nlo >= kFineNr ? 2 : 3, t0 = which * NT;
-            if (MODE == 1) {
-#pragma unroll
-                for (int k = 0; k < kTileLists; k++) list[k] += which == k ? np : 0;
-            }
+            const int n0 = c1 - c0 + 1, np = n0 + max(0, c3 - c2 + 1), which = list_of(h, nlo), t0 = which * NT;
+            tally(which, np);
+            if (MODE == 0) continue;
             // the columns of both ranges, four atomics on their way at a time
-            const int n0 = c1 - c0 + 1;
             for (int i = 0; i < np; i += 4) {
                 unsigned k[4];
                 int t[4];
