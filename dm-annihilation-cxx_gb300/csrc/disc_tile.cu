@@ -126,7 +126,9 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     return y;
 }
 
-// The exact FP64 chord test (and full rings).
+constexpr float kPiHi = 3.14159274101257324f, kPiLo = -8.74227765734758577e-8f;
+
+// The exact FP64 chord test.
 __device__ __noinline__ int exact_run(const DiscArgs &a, int q, int ring, int &lo, float &d0h) {
     const DiscHdr &d = a.chdr[q].hdr;
     int cnt;
@@ -166,6 +168,13 @@ __device__ __noinline__ int exact_run(const DiscArgs &a, int q, int ring, int &l
 template <bool GEN>
 __device__ __forceinline__ int tile_run(const DiscArgs &a, const TileHdr &h, const RingT &rc, int ring, int &lo,
                                         float &d0h, float &A, float &B) {
+    // nr phi0 / 2 pi - shift = fl + cf, fl an integer
+    auto split_phi = [&](float &fl, float &cf) {
+        const float hi = rc.nrf * h.ph;
+        const float lw = fmaf(rc.nrf, h.ph, -hi) + fmaf(rc.nrf, h.pl, -rc.shift);
+        fl = floorf(hi);
+        cf = (hi - fl) + lw;
+    };
     const float d = (rc.thh - h.t0h) + (rc.thl - h.t0l);
     float s;
     if (GEN) {
@@ -178,8 +187,18 @@ __device__ __forceinline__ int tile_run(const DiscArgs &a, const TileHdr &h, con
     }
     A = s * s;
     B = rc.st * h.sth0;
-    const bool chord = !GEN || !((h.flags & kFlagAll) || ring < h.irmin || ring > h.irmax);
-    if (chord && (h.flags & kFlagFast) && rc.st > 0.01f) {
+    if (GEN && ((h.flags & kFlagAll) || ring < h.irmin || ring > h.irmax)) {
+        // a full ring, from the pixel behind the antipodal azimuth on (FP32 may
+        // start it one pixel to the side of the FP64 form: the same pixels, the
+        // first at an offset of -pi / 2 to an ulp)
+        float fl, cf;
+        split_phi(fl, cf);
+        const float up = ceilf(cf);
+        lo = (int)fl + (int)up - rc.nr / 2;
+        d0h = fmaf(0.5f * rc.step, up - cf, -0.5f * kPiLo) - 0.5f * kPiHi;
+        return rc.nr;
+    }
+    if ((h.flags & kFlagFast) && rc.st > 0.01f) {
         const float num = h.hR - A;
         const float dnum = 7e-8f * h.hR + (GEN ? 7e-7f : 5.5e-7f) * A + 7e-8f * fabsf(num);
         if (num < -4.0f * dnum && -num > 1e-9f * B) return 0;   // clearly outside
@@ -202,10 +221,8 @@ __device__ __forceinline__ int tile_run(const DiscArgs &a, const TileHdr &h, con
             const float amp = GEN ? rsqrt_approx(1.0f - q) : 1.07f;
             const float ddphi = 1.05f * (eq * sq * amp + (GEN ? 4.5e-7f : 3.3e-7f) * dphi) +
                                 (GEN ? 1e-15f * (rB + rcp_approx(rc.st * rc.st)) : 4e-15f * rB) * rsq;
-            // nr phi0 / 2 pi - shift = fl + cf, fl an integer
-            const float hi = rc.nrf * h.ph;
-            const float lw = fmaf(rc.nrf, h.ph, -hi) + fmaf(rc.nrf, h.pl, -rc.shift);
-            const float fl = floorf(hi), cf = (hi - fl) + lw;
+            float fl, cf;
+            split_phi(fl, cf);
             const float w = rc.fnr * dphi;
             const float tau = rc.fnr * ddphi + 3e-7f * w + 6e-7f;
             const float xlo = cf - w, xhi = cf + w;
@@ -247,7 +264,6 @@ __device__ constexpr float kGwG[kNodesGen] = {1.279381961e-01f, 1.258374453e-01f
 __device__ constexpr float kGwGLo[kNodesGen] = {1.0278e-09f, 6.3130e-09f, 1.3962e-09f, -3.0681e-09f,
                                                 2.2970e-09f, 1.2565e-09f, 3.0315e-09f, 2.8634e-09f,
                                                 1.7837e-09f, 1.6689e-09f, -6.9250e-11f, 1.2575e-10f};
-constexpr float kPiHi = 3.14159274101257324f, kPiLo = -8.74227765734758577e-8f;
 constexpr int kDirect = 24, kDirectGen = 64;   // pixels up to which a ring is summed pixel by pixel
 constexpr int kFullPts = 32;                   // points of a full ring's trapezoid rule
 
