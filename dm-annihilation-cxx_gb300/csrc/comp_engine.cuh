@@ -366,7 +366,8 @@ __device__ inline float g_far(float x, const Run &r) {
 // g = theta^2 / 4.
 // TX, TH >= 0 fix the polynomial tiers at compile time (the disc kernels
 // dispatch on the particle's tiers once, outside the pixel loops); -1 reads
-// them from e.
+// them from e.  TH = 3 is tier 2 without the far hemisphere (h > 1/2: g is the
+// caller's to replace).
 template <int TX = -1, int TH = -1>
 __device__ __forceinline__ float2 exponent2x(const Ext &e, const Run &r, float2 jj, float2 &sn_out,
                                             float2 &h_out, float2 &g_out) {
@@ -405,8 +406,10 @@ __device__ __forceinline__ float2 exponent2x(const Ext &e, const Run &r, float2 
         g = mul2(h, q);
     } else {
         g = g_near2(make_float2(fmaxf(h.x, 0.0f), fmaxf(h.y, 0.0f)));
-        if (h.x > 0.5f) g.x = g_far(x.x, r);
-        if (h.y > 0.5f) g.y = g_far(x.y, r);
+        if (TH != 3) {
+            if (h.x > 0.5f) g.x = g_far(x.x, r);
+            if (h.y > 0.5f) g.y = g_far(x.y, r);
+        }
     }
     sn_out = sn;
     h_out = h;

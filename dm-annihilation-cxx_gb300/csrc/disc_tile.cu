@@ -1249,6 +1249,30 @@ __global__ void __launch_bounds__(kDepWarps * 32, kDepBlocks)
     }
 }
 
+// Exponents of eight consecutive pixels.  The far hemisphere's library calls
+// stand side by side: behind a branch per pixel each waited for the one before.
+__device__ __forceinline__ void exponents8(const Ext &e, const Run &r, float j, float2 (&t)[4]) {
+    float2 sn, h[4], g[4];
+    if (e.tier_h < 2) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) t[k] = exponent2x<-1, -1>(e, r, make_float2(j + 2 * k, j + 2 * k + 1), sn, h[k], g[k]);
+        return;
+    }
+    float top = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        t[k] = exponent2x<-1, 3>(e, r, make_float2(j + 2 * k, j + 2 * k + 1), sn, h[k], g[k]);
+        top = fmaxf(top, fmaxf(h[k].x, h[k].y));
+    }
+    if (!(top > 0.5f)) return;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 x = fma2(make_float2(j + 2 * k, j + 2 * k + 1), f2(r.steph), f2(r.d0h));
+        const float2 far = make_float2(g_far(x.x, r), g_far(x.y, r));
+        t[k] = mul2(make_float2(h[k].x > 0.5f ? far.x : g[k].x, h[k].y > 0.5f ? far.y : g[k].y), f2(e.nK));
+    }
+}
+
 constexpr int kGenWarps = 2;
 constexpr int kPxW = kTileW / 2;
 
@@ -1297,11 +1321,10 @@ __global__ void __launch_bounds__(kGenWarps * 32)
                 const int s = __reduce_min_sync(0xffffffffu, pc.s), end = __reduce_max_sync(0xffffffffu, pc.e);
                 for (int t = s; t < end; t += kStep) {
                     float2 wt[kStep / 2], wl[kStep / 2];   // w (F + Flo) as a two-float
+                    exponents8(e, r, (float)(t - pc.a), wl);
 #pragma unroll
                     for (int k = 0; k < kStep / 2; k++) {
-                        const float jf = (float)(t + 2 * k - pc.a);
-                        float2 sn, hv, g;
-                        const float2 wk = ex2_2(add2(exponent2x<-1, -1>(e, r, make_float2(jf, jf + 1.0f), sn, hv, g), sh2));
+                        const float2 wk = ex2_2(add2(wl[k], sh2));
                         wt[k] = mul2(wk, F2);
                         wl[k] = fma2(wk, Fl2, fma2(wk, F2, make_float2(-wt[k].x, -wt[k].y)));
                     }
