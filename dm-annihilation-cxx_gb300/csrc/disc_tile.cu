@@ -5,7 +5,7 @@
 // density those reductions bound a scatter (disc_seg.cu: 1.07e12 deposits/s
 // on the 16M-particle workload, 0.75 of a bare sweep of FP32 reductions).
 // Times below are of 1M of the 16M set's particles at Nside 2048 (4.6e10
-// deposits): 36 ms in all.  The whole set takes 0.60 s, and 1.22 s by the
+// deposits): 34 ms in all.  The whole set takes 0.54 s, and 1.16 s by the
 // segmented render.
 // Here a warp owns a tile of the map -- 32 rings (one per lane) by kTileW
 // in-ring pixel indices -- in registers, and walks the list of the discs
@@ -520,7 +520,7 @@ constexpr int kNormClaim = 4;   // discs per claim
 constexpr int kLongParts = 32;  // claims per general disc of more than kLongRings rings
 
 // S and the pixel count of every disc but the giants: a warp per disc, a ring
-// per lane.  5.6 ms, bound by FP32 issue (the ring's chord test and 8 or 12
+// per lane.  5.0 ms, bound by FP32 issue (the ring's chord test and 8 or 12
 // node values; the segmented render's first pass visits every pixel: 0.41 s
 // on the whole set).  A general disc of R = 2 at Nside 1522 has 3900 rings, 26 us
 // for each 32 of them: on one warp it took 2.9 ms, half of a map of 3000
@@ -1162,7 +1162,7 @@ __device__ __forceinline__ void for_items(const TileArgs &tg, const TileUnit &un
 // Units of one list: 0 and 1 polynomial discs (K_POLY3, K_POLY), 2 general
 // discs on fine rings, 3 the other general discs and the giants.  (Each list
 // has a kernel of its own: together they do not fit the instruction cache.)
-// Lists 0 to 2 take 19.5, 3.2 and 2.0 ms, the pixel kernel 0.8 ms.  Bound by
+// Lists 0 to 2 take 20.3, 3.4 and 2.2 ms, the pixel kernel 0.7 ms.  Bound by
 // issue (72 % of the slots): per (disc, tile) about 580 instructions -- a ring's
 // chord test per lane, then 3.5 instructions a pixel (exponent, ex2, the
 // predicated product) over the groups that any lane covers.
@@ -1250,7 +1250,8 @@ __global__ void __launch_bounds__(kDepWarps * 32, kDepBlocks)
 }
 
 // Exponents of eight consecutive pixels.  The far hemisphere's library calls
-// stand side by side: behind a branch per pixel each waited for the one before.
+// stand side by side: behind a branch per pixel each waited for the one before
+// (300 discs of R = 2.5 at Nside 1024: 16.9 -> 15.7 ms).
 __device__ __forceinline__ void exponents8(const Ext &e, const Run &r, float j, float2 (&t)[4]) {
     float2 sn, h[4], g[4];
     if (e.tier_h < 2) {
